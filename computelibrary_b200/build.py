@@ -62,9 +62,15 @@ def _compile_one(src: str, verbose: bool) -> str:
     return obj
 
 
+def _all_inputs() -> list[str]:
+    return [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [os.path.join(ROOT, "include", "cugl.h")]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every CUDA source (in parallel, one object each) and link one shared library; returns its path."""
     from concurrent.futures import ThreadPoolExecutor
+    if not force and os.path.exists(LIB_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(LIB_PATH) for d in _all_inputs()):
+        return LIB_PATH  # the library travels without its objects: nothing to recompile for
     os.makedirs(OBJ_DIR, exist_ok=True)
     if force:
         for f in os.listdir(OBJ_DIR):

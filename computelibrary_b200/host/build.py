@@ -115,12 +115,17 @@ def _link(objs: list[str], out: str, extra: list[str]) -> None:
         raise RuntimeError(f"g++ failed linking {out}")
 
 
+def prebuilt() -> bool:
+    """The three libraries are present from an earlier build on a machine with a Compute Library tree."""
+    return all(os.path.exists(p) for p in (LIB_PATH, ACL_HOST_LIB, GRAPH_LIB))
+
+
 def build(force: bool = False, acl_root: str | None = None) -> str:
     from computelibrary_b200 import build as cuda_build
     cuda_build.build()
     acl_root = acl_root or find_acl_root()
     if acl_root is None:
-        if os.path.exists(LIB_PATH) and os.path.exists(ACL_HOST_LIB) and os.path.exists(GRAPH_LIB):
+        if prebuilt():
             return LIB_PATH  # prebuilt libraries travel with the tree
         raise RuntimeError("no Compute Library tree (set ACL_ROOT) and no prebuilt libarm_compute_cuda.so")
     os.makedirs(OBJ_DIR, exist_ok=True)

@@ -12,6 +12,17 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run on the B200 box with -m gpu)")
 
 
+def pytest_collection_modifyitems(items):
+    # The C++ programs compile against a Compute Library tree; where there is neither a tree nor programs built
+    # beforehand on a machine that has one, there is nothing to run.
+    from computelibrary_b200.host import build as hb
+    if hb.find_acl_root() is not None or os.path.exists(os.path.join(ROOT, "tests", "cpp", "test_cu_functions")):
+        return
+    for item in items:
+        if os.path.basename(str(item.fspath)) == "test_host_cpp.py":
+            item.add_marker(pytest.mark.skip(reason="no Compute Library tree and no prebuilt C++ test programs"))
+
+
 @pytest.fixture(scope="session")
 def port():
     import oracle
