@@ -3,6 +3,8 @@
 // reshape.  All of them move each byte once with 128-bit accesses where the addresses allow it.
 #include "kernels.cuh"
 
+#include <climits>
+
 namespace cugl
 {
 namespace
@@ -25,6 +27,34 @@ __device__ __forceinline__ int32_t warp_sum(int32_t v)
     return v;
 }
 
+// A warp's share of the byte sum of n 16-byte vectors: four independent loads in flight per lane.
+__device__ __forceinline__ int32_t sum_vectors(const uint4 *v, int n, int lane, bool is_signed, int32_t acc)
+{
+    int i = lane;
+    for (; i + 96 < n; i += 128)
+    {
+        const uint4 q0 = __ldg(v + i), q1 = __ldg(v + i + 32), q2 = __ldg(v + i + 64), q3 = __ldg(v + i + 96);
+        int32_t     a0 = sum4(q0.x, is_signed, 0), a1 = sum4(q1.x, is_signed, 0);
+        int32_t     a2 = sum4(q2.x, is_signed, 0), a3 = sum4(q3.x, is_signed, 0);
+        a0 = sum4(q0.y, is_signed, a0), a1 = sum4(q1.y, is_signed, a1);
+        a2 = sum4(q2.y, is_signed, a2), a3 = sum4(q3.y, is_signed, a3);
+        a0 = sum4(q0.z, is_signed, a0), a1 = sum4(q1.z, is_signed, a1);
+        a2 = sum4(q2.z, is_signed, a2), a3 = sum4(q3.z, is_signed, a3);
+        a0 = sum4(q0.w, is_signed, a0), a1 = sum4(q1.w, is_signed, a1);
+        a2 = sum4(q2.w, is_signed, a2), a3 = sum4(q3.w, is_signed, a3);
+        acc += (a0 + a1) + (a2 + a3);
+    }
+    for (; i < n; i += 32)
+    {
+        const uint4 q = __ldg(v + i);
+        acc           = sum4(q.x, is_signed, acc);
+        acc           = sum4(q.y, is_signed, acc);
+        acc           = sum4(q.z, is_signed, acc);
+        acc           = sum4(q.w, is_signed, acc);
+    }
+    return acc;
+}
+
 // ---- rowsum_A[m] = scalar * sum_k A[m,k] -------------------------------------------------------
 // One warp per row: unaligned head bytes, a body of 16-byte vectors, tail bytes; shuffle reduction.
 // CpuGemmLowpMatrixAReductionKernel::run_internal (CpuGemmLowpMatrixReductionKernel.cpp:133-204).
@@ -43,30 +73,8 @@ __global__ void __launch_bounds__(kThreads) reduce_rows_kernel(const uint8_t *__
         {
             acc += load_q8(row, lane, is_signed);
         }
-        const int    nvec = (K - head) >> 4;
-        const uint4 *v    = reinterpret_cast<const uint4 *>(row + head);
-        int i = lane;
-        for (; i + 96 < nvec; i += 128) // four independent 16-byte loads in flight per lane
-        {
-            const uint4 q0 = __ldg(v + i), q1 = __ldg(v + i + 32), q2 = __ldg(v + i + 64), q3 = __ldg(v + i + 96);
-            int32_t     a0 = sum4(q0.x, is_signed, 0), a1 = sum4(q1.x, is_signed, 0);
-            int32_t     a2 = sum4(q2.x, is_signed, 0), a3 = sum4(q3.x, is_signed, 0);
-            a0 = sum4(q0.y, is_signed, a0), a1 = sum4(q1.y, is_signed, a1);
-            a2 = sum4(q2.y, is_signed, a2), a3 = sum4(q3.y, is_signed, a3);
-            a0 = sum4(q0.z, is_signed, a0), a1 = sum4(q1.z, is_signed, a1);
-            a2 = sum4(q2.z, is_signed, a2), a3 = sum4(q3.z, is_signed, a3);
-            a0 = sum4(q0.w, is_signed, a0), a1 = sum4(q1.w, is_signed, a1);
-            a2 = sum4(q2.w, is_signed, a2), a3 = sum4(q3.w, is_signed, a3);
-            acc += (a0 + a1) + (a2 + a3);
-        }
-        for (; i < nvec; i += 32)
-        {
-            const uint4 q = __ldg(v + i);
-            acc           = sum4(q.x, is_signed, acc);
-            acc           = sum4(q.y, is_signed, acc);
-            acc           = sum4(q.z, is_signed, acc);
-            acc           = sum4(q.w, is_signed, acc);
-        }
+        const int nvec = (K - head) >> 4;
+        acc            = sum_vectors(reinterpret_cast<const uint4 *>(row + head), nvec, lane, is_signed, acc);
         const int tail0 = head + (nvec << 4);
         if (tail0 + lane < K)
         {
@@ -156,102 +164,218 @@ __global__ void scale_vector_kernel(int32_t *v, int n, int32_t scalar)
     }
 }
 
-// ---- prepare(): B [K,N] (N contiguous) -> Bt [N, ldbt] (K contiguous) + column sums -------------
-// 64 x 64 byte tiles through shared memory: reads are coalesced along N, writes along K.  Each block
-// also reduces its 64 rows per column and adds the partial sums with integer atomics, so B is read
-// exactly once for both products of prepare().  colsum (when not null) must be zero on entry.
-__global__ void __launch_bounds__(kThreads) transpose_colsum_kernel(const uint8_t *__restrict__ b, bool is_signed,
-                                                                    int K, int N, int64_t ldb,
-                                                                    uint8_t *__restrict__ bt, int64_t ldbt,
-                                                                    int32_t *__restrict__ colsum)
+// ---- operand preparation ---------------------------------------------------------------------------------
+// One launch does everything the tensor-core kernel needs from its operands beforehand, for all products of a batch:
+// blocks [0, b_blocks) turn B [K][N] (N contiguous) into Bt [N][ldbt] (K contiguous) with its column sums, the blocks
+// behind them walk over the rows of A and produce row sums and, where the TMA engine cannot address A (base or pitch
+// not a multiple of 16 bytes), a copy with 16-byte rows.  The work is bound by launches when the operands are small
+// (16 products of 384 x 384 x 128 with a B that changes took 64 launches one after the other, 229 us; with this launch
+// and a batched product 10.3 us.  923 x 429 x 873 with unaligned rows: copy + reduction + product 24.6 us, now 20.1) and
+// by HBM when they are large.
+struct PrepParams
 {
-    __shared__ uint8_t tile[64][64 + 4];
-    const int          k0 = blockIdx.y * 64;
-    const int          n0 = blockIdx.x * 64;
-    const int          tx = threadIdx.x & 63; // fastest index
-    const int          ty = threadIdx.x >> 6; // 0..3
-#pragma unroll 4
-    for (int r = ty; r < 64; r += 4)
+    OperandPrep op;
+    int         b_strips, b_splits, b_blocks, k_per_split; // strips of 64 columns, K splits of k_per_split rows
+    int         row_lanes; // lanes that share a row of A
+    bool        b_words, a_vec; // B rows 4-byte aligned / A rows 16-byte aligned
+};
+
+// Four consecutive bytes starting at p, of which `valid` (>= 1) exist; the rest read as zero.
+__device__ __forceinline__ uint32_t load_bytes4(const uint8_t *p, int valid)
+{
+    uint32_t v = p[0];
+    if (valid > 1) v |= static_cast<uint32_t>(p[1]) << 8;
+    if (valid > 2) v |= static_cast<uint32_t>(p[2]) << 16;
+    if (valid > 3) v |= static_cast<uint32_t>(p[3]) << 24;
+    return v;
+}
+
+// B: a block owns 64 columns and a range of K and walks down it 128 rows at a time.  A thread reads 4 x 4 bytes (four
+// rows of one 32-bit column word), transposes them with eight byte permutes and leaves four K-contiguous words in
+// shared memory; the tile goes out as 128 contiguous bytes per column.  The column sums come from the transposed words
+// (__dp4a); with one split per strip they are plain stores, else integer atomics on zeroed sums (exact in any order).
+__device__ __forceinline__ void prepare_b_strip(const PrepParams &p, int block, uint32_t (*tile)[33])
+{
+    const OperandPrep &o     = p.op;
+    const int          split = block % p.b_splits, sz = block / p.b_splits;
+    const int          strip = sz % p.b_strips, z = sz / p.b_strips;
+    const int          n0 = strip * 64, k_begin = split * p.k_per_split, k_end = min(o.K, k_begin + p.k_per_split);
+    const uint8_t     *b  = o.b + z * o.b_batch_stride;
+    uint8_t           *bt = o.bt + static_cast<int64_t>(z) * o.N * o.ldbt;
+    const int          w = threadIdx.x & 15, g = threadIdx.x >> 4; // column word, group of four rows (of 16)
+    const int          n = n0 + 4 * w;
+    const int          piece = threadIdx.x & 7, col = threadIdx.x >> 3; // output: eight threads write 128 bytes of a column
+    int32_t            sum[2] = {0, 0}; // columns col, col + 32 of the strip: this thread's share
+    for (int k0 = k_begin; k0 < k_end; k0 += 128)
     {
-        const int k = k0 + r, n = n0 + tx;
-        tile[r][tx] = (k < K && n < N) ? b[static_cast<int64_t>(k) * ldb + n] : 0;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int r = ty; r < 64; r += 4)
-    {
-        const int n = n0 + r, k = k0 + tx;
-        if (n < N && k < K)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
         {
-            bt[static_cast<int64_t>(n) * ldbt + k] = tile[tx][r];
-        }
-    }
-    if (colsum != nullptr && threadIdx.x < 64)
-    {
-        const int n = n0 + threadIdx.x;
-        if (n < N)
-        {
-            int32_t s = 0;
-#pragma unroll 8
-            for (int r = 0; r < 64; ++r)
+            const int kg = g + 16 * h, k = k0 + 4 * kg;
+            uint32_t  r[4] = {0, 0, 0, 0};
+            if (n < o.N)
             {
-                const uint8_t v = tile[r][threadIdx.x];
-                s += is_signed ? static_cast<int32_t>(static_cast<int8_t>(v)) : static_cast<int32_t>(v);
+                const uint8_t *src = b + static_cast<int64_t>(k) * o.ldb + n;
+                if (p.b_words && n + 4 <= o.N)
+                {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (k + i < k_end) r[i] = __ldg(reinterpret_cast<const uint32_t *>(src + i * o.ldb));
+                }
+                else
+                {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (k + i < k_end) r[i] = load_bytes4(src + i * o.ldb, o.N - n);
+                }
             }
-            atomicAdd(colsum + n, s);
+            const uint32_t a0 = __byte_perm(r[0], r[1], 0x5140), a1 = __byte_perm(r[2], r[3], 0x5140);
+            const uint32_t b0 = __byte_perm(r[0], r[1], 0x7362), b1 = __byte_perm(r[2], r[3], 0x7362);
+            // column c of the strip, K word kg: row c of `tile`, 33 words apart
+            tile[4 * w + 0][kg] = __byte_perm(a0, a1, 0x5410);
+            tile[4 * w + 1][kg] = __byte_perm(a0, a1, 0x7632);
+            tile[4 * w + 2][kg] = __byte_perm(b0, b1, 0x5410);
+            tile[4 * w + 3][kg] = __byte_perm(b0, b1, 0x7632);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+        {
+            const int       c  = col + 32 * h;
+            const uint32_t *tw = &tile[c][4 * piece];
+            const uint4     v  = make_uint4(tw[0], tw[1], tw[2], tw[3]);
+            sum[h] = sum4(v.x, o.b_signed, sum[h]);
+            sum[h] = sum4(v.y, o.b_signed, sum[h]);
+            sum[h] = sum4(v.z, o.b_signed, sum[h]);
+            sum[h] = sum4(v.w, o.b_signed, sum[h]);
+            // ldbt is a multiple of 128: what the tile holds beyond K is the zero padding of the row
+            if (n0 + c < o.N)
+            {
+                *reinterpret_cast<uint4 *>(bt + static_cast<int64_t>(n0 + c) * o.ldbt + k0 + 16 * piece) = v;
+            }
+        }
+        __syncthreads();
+    }
+    if (o.colsum != nullptr)
+    {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+        {
+            int32_t s = sum[h];
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            s += __shfl_xor_sync(0xffffffffu, s, 4);
+            const int c = n0 + col + 32 * h;
+            if (piece == 0 && c < o.N)
+            {
+                int32_t *out = o.colsum + static_cast<int64_t>(z) * o.N + c;
+                if (p.b_splits == 1) *out = s;
+                else atomicAdd(out, s);
+            }
         }
     }
 }
 
-// The same with 32-bit global accesses (four bytes per thread and instruction instead of one): K, N, both pitches and
-// both base addresses multiples of 4.  A 64 x 64 tile is loaded as 16 words per row, transposed byte by byte out of
-// shared memory (four byte reads and three permutes per output word) and stored as 16 words per output row.
-__global__ void __launch_bounds__(kThreads) transpose_colsum_words_kernel(const uint8_t *__restrict__ b, bool is_signed,
-                                                                          int K, int N, int64_t ldb,
-                                                                          uint8_t *__restrict__ bt, int64_t ldbt,
-                                                                          int32_t *__restrict__ colsum)
+// A: 16 bytes per lane and step, as many lanes to a row as it has such pieces (a power of two, at most the warp; the
+// pixels of a convolution input are rows of a few pieces).  A row that is not 16-byte aligned is read as five aligned
+// words and shifted into place (the words of neighbouring lanes overlap and hit L1); the two ends of such a row, whose
+// aligned words reach outside it, are read byte by byte.
+__device__ __forceinline__ uint4 load_row16(const uint8_t *row, int k, int K, bool vec)
 {
-    __shared__ uint32_t tile[64][16 + 1]; // [k][n / 4], one word of padding per row
-    const int           k0 = blockIdx.y * 64;
-    const int           n0 = blockIdx.x * 64;
-    const int           w  = threadIdx.x & 15; // word of the row
-    const int           r4 = threadIdx.x >> 4; // 0..15
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
+    const uint8_t *p = row + k;
+    const int      o = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 3);
+    if (k + 16 <= K && vec)
     {
-        const int r = r4 + 16 * i, k = k0 + r, n = n0 + 4 * w;
-        tile[r][w]  = (k < K && n < N) ? __ldg(reinterpret_cast<const uint32_t *>(b + static_cast<int64_t>(k) * ldb + n)) : 0u;
+        return __ldg(reinterpret_cast<const uint4 *>(p));
     }
-    __syncthreads();
-    const uint8_t *bytes = reinterpret_cast<const uint8_t *>(&tile[0][0]);
-    constexpr int  kPitch = (16 + 1) * 4; // bytes per tile row
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
+    if (k + 16 <= K && o == 0)
     {
-        const int n = r4 + 16 * i, k = k0 + 4 * w; // output row n0 + n, output word w: bytes tile[4w .. 4w+3][n]
-        if (n0 + n < N && k < K)
-        {
-            const uint32_t v = static_cast<uint32_t>(bytes[(4 * w + 0) * kPitch + n]) |
-                               (static_cast<uint32_t>(bytes[(4 * w + 1) * kPitch + n]) << 8) |
-                               (static_cast<uint32_t>(bytes[(4 * w + 2) * kPitch + n]) << 16) |
-                               (static_cast<uint32_t>(bytes[(4 * w + 3) * kPitch + n]) << 24);
-            *reinterpret_cast<uint32_t *>(bt + static_cast<int64_t>(n0 + n) * ldbt + k) = v;
-        }
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(p);
+        return make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
     }
-    if (colsum != nullptr && threadIdx.x < 64)
+    if (k >= 4 && k + 20 <= K) // the aligned words of [k - o, k - o + 20) lie inside the row
     {
-        const int n = n0 + threadIdx.x;
-        if (n < N)
+        const uint32_t *w  = reinterpret_cast<const uint32_t *>(p - o);
+        const uint32_t  w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3), w4 = __ldg(w + 4);
+        return make_uint4(__funnelshift_r(w0, w1, 8 * o), __funnelshift_r(w1, w2, 8 * o), __funnelshift_r(w2, w3, 8 * o),
+                          __funnelshift_r(w3, w4, 8 * o));
+    }
+    uint32_t v[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+        if (k + 4 * j < K) v[j] = load_bytes4(p + 4 * j, K - k - 4 * j);
+    }
+    return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+__device__ __forceinline__ void prepare_a_rows(const PrepParams &p, int block, int n_blocks)
+{
+    const OperandPrep &o    = p.op;
+    const int          lane = threadIdx.x & 31;
+    const int          sub  = lane & (p.row_lanes - 1), per_warp = 32 / p.row_lanes;
+    const int          k_all = o.copy != nullptr ? static_cast<int>(o.kp) : o.K; // what a row's sum covers
+    const int64_t      rows = static_cast<int64_t>(o.rows) * o.batch_a;
+    for (int64_t m0 = (static_cast<int64_t>(block) * (kThreads / 32) + (threadIdx.x >> 5)) * per_warp; m0 < rows;
+         m0 += static_cast<int64_t>(n_blocks) * (kThreads / 32) * per_warp)
+    {
+        const int64_t m   = m0 + lane / p.row_lanes; // (lanes of a row beyond the last one only take part in the sum)
+        int32_t       acc = 0;
+        if (m < rows)
         {
-            int32_t s = 0;
-#pragma unroll 8
-            for (int r = 0; r < 64; ++r)
+            const int64_t  z   = o.batch_a > 1 ? m / o.rows : 0;
+            const uint8_t *row = o.a + z * o.a_batch_stride + (m - z * o.rows) * o.lda;
+            uint8_t       *out = o.copy != nullptr ? o.copy + m * o.kp : nullptr;
+            int            k   = 16 * sub;
+            if (p.a_vec && out == nullptr && p.row_lanes == 32) // long aligned rows, sums only
             {
-                const uint8_t v = bytes[r * kPitch + threadIdx.x];
-                s += is_signed ? static_cast<int32_t>(static_cast<int8_t>(v)) : static_cast<int32_t>(v);
+                acc = sum_vectors(reinterpret_cast<const uint4 *>(row), o.K >> 4, lane, o.a_signed, 0);
+                k   = (o.K >> 4) * 16 + 16 * sub; // the piece beyond the last whole one
             }
-            atomicAdd(colsum + n, s);
+#pragma unroll 4
+            for (; k < k_all; k += 16 * p.row_lanes)
+            {
+                uint4 v = load_row16(row, k, o.K, p.a_vec);
+                if (o.fill != 0 && k + 16 > o.K) // bytes K .. kp - 1
+                {
+                    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                    {
+                        if (k + j >= o.K) w[j >> 2] |= static_cast<uint32_t>(o.fill) << (8 * (j & 3));
+                    }
+                    v = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+                if (out != nullptr) *reinterpret_cast<uint4 *>(out + k) = v;
+                acc = sum4(v.x, o.a_signed, acc);
+                acc = sum4(v.y, o.a_signed, acc);
+                acc = sum4(v.z, o.a_signed, acc);
+                acc = sum4(v.w, o.a_signed, acc);
+            }
         }
+        if (o.rowsum != nullptr)
+        {
+            for (int x = p.row_lanes >> 1; x > 0; x >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, x);
+            if (sub == 0 && m < rows) o.rowsum[m] = acc;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) prepare_operands_kernel(const __grid_constant__ PrepParams p)
+{
+    __shared__ uint32_t tile[64][33];
+    // the tensor-core kernel behind this launch may set itself up meanwhile; this kernel itself touches memory only
+    // after everything before it in the stream has completed
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int block = static_cast<int>(blockIdx.x);
+    if (block < p.b_blocks)
+    {
+        prepare_b_strip(p, block, tile);
+    }
+    else
+    {
+        prepare_a_rows(p, block - p.b_blocks, static_cast<int>(gridDim.x) - p.b_blocks);
     }
 }
 
@@ -634,28 +758,55 @@ cugl_status launch_reduce_cols(cugl_context *ctx, const void *d_b, bool is_signe
     return CUGL_SUCCESS;
 }
 
-cugl_status launch_transpose_colsum(cugl_context *ctx, const void *d_b, bool is_signed, int K, int N, int64_t ldb,
-                                    void *d_bt, int64_t ldbt, int32_t *d_colsum)
+cugl_status launch_prepare_operands(cugl_context *ctx, const OperandPrep &op)
 {
-    if (d_colsum != nullptr)
+    PrepParams p{};
+    p.op = op;
+    if (op.b != nullptr && op.N > 0 && op.K > 0)
     {
-        CUGL_CUDA_TRY(ctx, cudaMemsetAsync(d_colsum, 0, sizeof(int32_t) * N, ctx->stream));
+        // One strip of 64 columns per block, all of K, when the strips alone give every SM a block: the column sums then
+        // need neither zeroed memory nor atomics.  Else K is split until about two blocks per SM exist.
+        p.b_strips = (op.N + 63) / 64;
+        const int64_t strips = static_cast<int64_t>(p.b_strips) * op.batch_b;
+        const int64_t k_tiles = (op.K + 127) / 128;
+        int64_t splits = strips >= ctx->sm_count ? 1 : (2 * ctx->sm_count + strips - 1) / strips;
+        splits         = splits < k_tiles ? splits : k_tiles;
+        if (k_tiles <= 4) splits = 1; // a strip of a few tiles is finished sooner than a memset and its launch
+        const int64_t tiles_per_split = (k_tiles + splits - 1) / splits;
+        p.k_per_split = static_cast<int>(tiles_per_split * 128);
+        p.b_splits    = static_cast<int>((k_tiles + tiles_per_split - 1) / tiles_per_split);
+        const int64_t blocks = strips * p.b_splits;
+        if (blocks > INT32_MAX / 2) return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "B operand: too many column strips");
+        p.b_blocks = static_cast<int>(blocks);
+        p.b_words  = ((reinterpret_cast<uintptr_t>(op.b) | static_cast<uint64_t>(op.ldb) |
+                       static_cast<uint64_t>(op.batch_b > 1 ? op.b_batch_stride : 0)) & 3) == 0;
+        if (p.b_splits > 1 && op.colsum != nullptr)
+        {
+            CUGL_CUDA_TRY(ctx, cudaMemsetAsync(op.colsum, 0, sizeof(int32_t) * static_cast<size_t>(op.N) * op.batch_b, ctx->stream));
+        }
     }
-    if (K <= 0 || N <= 0) return CUGL_SUCCESS;
-    dim3 grid((N + 63) / 64, (K + 63) / 64);
-    const uint64_t bits = reinterpret_cast<uintptr_t>(d_b) | reinterpret_cast<uintptr_t>(d_bt) | static_cast<uint64_t>(ldb) |
-                          static_cast<uint64_t>(ldbt) | static_cast<uint64_t>(K) | static_cast<uint64_t>(N);
-    if ((bits & 3) == 0)
+    int a_blocks = 0;
+    if (op.a != nullptr && op.rows > 0)
     {
-        transpose_colsum_words_kernel<<<grid, kThreads, 0, ctx->stream>>>(static_cast<const uint8_t *>(d_b), is_signed, K, N,
-                                                                          ldb, static_cast<uint8_t *>(d_bt), ldbt, d_colsum);
+        p.a_vec = ((reinterpret_cast<uintptr_t>(op.a) | static_cast<uint64_t>(op.lda) |
+                    static_cast<uint64_t>(op.batch_a > 1 ? op.a_batch_stride : 0)) & 15) == 0;
+        p.row_lanes = 1;
+        while (p.row_lanes < 32 && p.row_lanes * 16 < op.K) p.row_lanes *= 2;
+        a_blocks = grid_for(static_cast<int64_t>(op.rows) * op.batch_a * p.row_lanes, ctx->sm_count);
     }
-    else
-    {
-        transpose_colsum_kernel<<<grid, kThreads, 0, ctx->stream>>>(static_cast<const uint8_t *>(d_b), is_signed, K, N,
-                                                                    ldb, static_cast<uint8_t *>(d_bt), ldbt, d_colsum);
-    }
-    return check_cuda(ctx, cudaGetLastError(), "transpose_colsum_kernel");
+    if (p.b_blocks + a_blocks == 0) return CUGL_SUCCESS;
+    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, prepare_operands_kernel, p.b_blocks + a_blocks, kThreads, 0, p));
+    return check_cuda(ctx, cudaGetLastError(), "prepare_operands_kernel");
+}
+
+cugl_status launch_transpose_colsum(cugl_context *ctx, const void *d_b, bool is_signed, int K, int N, int64_t ldb,
+                                    void *d_bt, int64_t ldbt, int32_t *d_colsum, int batch, int64_t b_batch_stride)
+{
+    OperandPrep op{};
+    op.b = static_cast<const uint8_t *>(d_b), op.ldb = ldb, op.b_batch_stride = b_batch_stride;
+    op.bt = static_cast<uint8_t *>(d_bt), op.ldbt = ldbt, op.colsum = d_colsum, op.b_signed = is_signed;
+    op.N = N, op.K = K, op.batch_b = batch;
+    return launch_prepare_operands(ctx, op);
 }
 
 cugl_status launch_transpose_bytes(cugl_context *ctx, const void *d_src, int rows, int cols, void *d_dst, int batch)

@@ -36,7 +36,7 @@ int pick_block_n(const cugl_context *ctx, const GemmOperands &op)
         return widest; // kernels the caller asked for by name: 256-column tiles only
     }
     const long long sms     = ctx->sm_count > 0 ? ctx->sm_count : 1;
-    const long long m_tiles = (op.M + 127) / 128;
+    const long long m_tiles = static_cast<long long>((op.M + 127) / 128) * (op.batch > 1 ? op.batch : 1);
     if (m_tiles * ((op.N + widest - 1) / widest) >= sms)
     {
         return widest;
@@ -91,6 +91,12 @@ cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, c
     // 57 / 60; 12544 x 2048 x 512: 37 / 43.  It needs whole 128-channel blocks (N = 64: 110 / 78).
     GemmOperands o   = op;
     o.block_n        = pick_block_n(ctx, op); // before the automatic channel-major choice below
+    if (op.batch > 1)
+    {
+        // Batches of attention-sized products: their tiles share one grid instead of each product filling its own
+        // (16 products of 384 x 384 x 128: 6 - 18 tiles each).
+        return launch_gemmlowp_tcgen05_epi8(ctx, o, ep, false);
+    }
     if (ep.stage == CUGL_STAGE_NONE && (ep.out_f32 != 0 || ep.accumulate != 0) && o.channel_major == 0)
     {
         o.channel_major = -1; // read-modify-write of dst rows: the row-major epilogue does it with 128-bit accesses

@@ -27,6 +27,8 @@
 
 #include <cuda.h>
 
+#include <climits>
+
 namespace cugl
 {
 namespace
@@ -189,6 +191,20 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t sr
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
                  :
                  : "l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 :
+                 : "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, uint32_t src, int c0, int c1, int c2)
+{
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
+                 :
+                 : "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(src)
                  : "memory");
 }
 __device__ __forceinline__ void tma_store_commit()
@@ -391,6 +407,11 @@ struct TileParams
     // fill value of out-of-image taps), and for C a multiple of 128.
     int      conv_c, conv_kw, conv_wo, conv_ho, conv_sx, conv_sy, conv_pl, conv_pt, conv_dx, conv_dy;
     FastDiv  conv_div_wo, conv_div_ho;
+    // Batched product (kBatched instantiations): `batch` equal products in one launch, operand and output maps with a third
+    // dimension.  Strides in elements of what they advance: bytes of dst, entries of the column and row sums.
+    int      batch;
+    int64_t  batch_dst;
+    int      batch_colsum, batch_rowsum;
     int      tma_store;               // one-CTA row-major kernels: staged groups leave as bulk tensor stores (tmap_out)
     long long spin_limit;             // clock64 ticks a wait on a barrier may last before the kernel gives up
     int      withhold_kb;             // >= 0: CTA 0 leaves out the copies of this k-block ordinal (test instrument
@@ -693,7 +714,7 @@ __device__ __forceinline__ void stage_chunk(uint8_t *stage, const uint32_t *w, i
 }
 
 __device__ __forceinline__ void flush_stage(const uint8_t *stage, const TileParams &tp, int m_base, int n_group,
-                                            int ncols_group, int lane, bool tma = false)
+                                            int ncols_group, int lane, bool tma = false, int64_t dst_off = 0)
 {
     __syncwarp();
     const int p = lane & (kOutPieces - 1);
@@ -706,7 +727,7 @@ __device__ __forceinline__ void flush_stage(const uint8_t *stage, const TilePara
         if (p * 16 < ncols_group && m < tp.M && n < tp.N)
         {
             const uint4   val = *reinterpret_cast<const uint4 *>(stage + r * kOutRowBytes + ((p ^ stage_sw(r, tma)) << 4));
-            const int64_t off = static_cast<int64_t>(m) * tp.ldd + n;
+            const int64_t off = dst_off + static_cast<int64_t>(m) * tp.ldd + n;
             if (n + 16 <= tp.N && tp.vec_ok)
             {
                 *reinterpret_cast<uint4 *>(tp.dst + off) = val;
@@ -738,13 +759,14 @@ __device__ __forceinline__ void flush_stage(const uint8_t *stage, const TilePara
 // not make it wait for the stores to be accepted.  The caller waits for the previous group's reads (stage_reuse_wait)
 // before it writes into the stage again.
 __device__ __forceinline__ void flush_stage_tma(const uint8_t *stage, const CUtensorMap *omap, int m_base, int n_group,
-                                                int lane)
+                                                int lane, int z = -1)
 {
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0)
     {
-        tma_store_2d(omap, smem_u32(stage), n_group, m_base);
+        if (z >= 0) tma_store_3d(omap, smem_u32(stage), n_group, m_base, z); // batched map
+        else tma_store_2d(omap, smem_u32(stage), n_group, m_base);
         tma_store_commit();
     }
 }
@@ -849,10 +871,11 @@ template <int NCOLS, bool kS32Out, int kMode>
 __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s_col, const TileParams &tp,
                                                   const EpilogueParams &ep, int m, int n_first, int32_t row_term,
                                                   uint8_t *stage, int lane, const AccRelease &rel,
-                                                  const CUtensorMap *omap = nullptr)
+                                                  const CUtensorMap *omap = nullptr, int z = -1)
 {
     const bool row_ok = m < tp.M;
-    const int64_t row_off = static_cast<int64_t>(m) * tp.ldd;
+    const int64_t dst_off = z >= 0 ? z * tp.batch_dst : 0; // z: which product of a batched launch, -1 outside one
+    const int64_t row_off = dst_off + static_cast<int64_t>(m) * tp.ldd;
     uint8_t      *drow    = tp.dst + row_off;
     // omap: the warp's 32 rows x kOutRowBytes leave as one bulk tensor store from its staging area (one destination)
     const bool    tma     = !kS32Out && omap != nullptr && tp.n_extra == 0; // warp-uniform
@@ -875,11 +898,11 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
             const int n_group = n_first + first * 32;
             if (tma && ncols == kOutRowBytes && (n_group + kOutRowBytes <= tp.N || (tp.N & 15) == 0))
             {
-                flush_stage_tma(stage, omap, m - lane, n_first + first * 32, lane);
+                flush_stage_tma(stage, omap, m - lane, n_first + first * 32, lane, z);
             }
             else
             {
-                flush_stage(stage, tp, m - lane, n_first + first * 32, ncols, lane, tma);
+                flush_stage(stage, tp, m - lane, n_first + first * 32, ncols, lane, tma, dst_off);
             }
         }
     };
@@ -1601,7 +1624,7 @@ template <int BLOCK_N, bool kS32Out, int kGroups = 1>
 __device__ __forceinline__ void epilogue_warp_tile(uint32_t tmem_acc, const int4 *s_col, const TileParams &tp,
                                                    const EpilogueParams &ep, int warp, int lane, int m0, int n0,
                                                    uint8_t *out_stage, const AccRelease &rel,
-                                                   const CUtensorMap *omap = nullptr)
+                                                   const CUtensorMap *omap = nullptr, int z = -1)
 {
     constexpr int NCOLS    = BLOCK_N * kGroups / (kEpiWarps / 4);
     uint8_t      *stage    = out_stage + (warp - kFirstEpi) * kOutStageBytes;
@@ -1613,27 +1636,27 @@ __device__ __forceinline__ void epilogue_warp_tile(uint32_t tmem_acc, const int4
     if (tp.mode == kStagePack && !kS32Out)
     {
         drain_accumulator<NCOLS, kS32Out, kStagePack>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
-                                                      stage, lane, rel, omap);
+                                                      stage, lane, rel, omap, z);
     }
     else if (tp.mode == kStagePackS && !kS32Out)
     {
         drain_accumulator<NCOLS, kS32Out, kStagePackS>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
-                                                       stage, lane, rel, omap);
+                                                       stage, lane, rel, omap, z);
     }
     else if (tp.mode == kStageWide && !kS32Out)
     {
         drain_accumulator<NCOLS, kS32Out, kStageWide>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
-                                                      stage, lane, rel, omap);
+                                                      stage, lane, rel, omap, z);
     }
     else if (tp.mode == kStageGeneric)
     {
         drain_accumulator<NCOLS, kS32Out, kStageGeneric>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS,
-                                                         row_term, stage, lane, rel, omap);
+                                                         row_term, stage, lane, rel, omap, z);
     }
     else
     {
         drain_accumulator<NCOLS, kS32Out, kStageFast>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
-                                                      stage, lane, rel, omap);
+                                                      stage, lane, rel, omap, z);
     }
 }
 
@@ -1673,7 +1696,10 @@ struct SmemPlan
 // activation matrix, tp.M the number of output channels and tp.N the number of output rows -- so the
 // accumulator holds the transposed output tile and epilogue_warp_tile_cm writes it (see there).  Tiles are then
 // ordered n-fastest, i.e. all row blocks of one channel block in turn.
-template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kCM, int ACC, bool kPairTma = false>
+// kBatched: tp.batch equal products in one launch.  A tile index then runs over (product, column block, row block),
+// row blocks fastest, so the column terms still carry over from tile to tile; operands and bulk stores go through
+// three-dimensional tensor maps, whose bounds keep a ragged last row block inside its own product.
+template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kCM, int ACC, bool kPairTma = false, bool kBatched = false>
 __global__ void __launch_bounds__(kThreads, 1)
     gemmlowp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                             const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_res,
@@ -1702,7 +1728,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     const int num_m_blocks = (tp.M + BLOCK_M - 1) / BLOCK_M;
     const int num_n_blocks = (tp.N + BLOCK_N - 1) / BLOCK_N;
-    const int num_tiles    = num_m_blocks * num_n_blocks;
+    const int num_tiles    = num_m_blocks * num_n_blocks * (kBatched ? tp.batch : 1);
+    static_assert(!(kBatched && (kCM || kPairTma)), "batched launches use the row-major single-tile drain");
     const int num_kb       = (tp.K + KSUB * BLOCK_K - 1) / (KSUB * BLOCK_K); // pipeline stages per tile
 
     if (threadIdx.x == 0)
@@ -1771,9 +1798,24 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 const int tile = static_cast<int>(blockIdx.x) + ti * static_cast<int>(gridDim.x);
                 const int m0   = (kCM ? tile / num_n_blocks : tile % num_m_blocks) * BLOCK_M;
-                const int n0   = (kCM ? tile % num_n_blocks : tile / num_m_blocks) * BLOCK_N;
+                const int nb   = kCM ? tile % num_n_blocks : tile / num_m_blocks;
+                const int z    = kBatched ? nb / num_n_blocks : 0;
+                const int n0   = (kBatched ? nb - z * num_n_blocks : nb) * BLOCK_N;
                 if (kb == 0) trace_event(tp.trace, ti, 0);
-                if (!kCM && tp.conv_c != 0)
+                if (kBatched)
+                {
+                    mbar_expect_tx(full_bar(st), P::STAGE);
+#pragma unroll
+                    for (int sub = 0; sub < KSUB; ++sub)
+                    {
+                        const int k0 = (kb * KSUB + sub) * BLOCK_K;
+                        tma_load_3d(sA + st * P::A_STAGE_K + sub * A_STAGE, &tmap_a, k0, m0, z, full_bar(st));
+                        tma_load_3d(sB + st * P::B_STAGE + sub * P::B_SUB, &tmap_b, k0, n0, tp.batch_colsum != 0 ? z : 0, full_bar(st));
+                    }
+                    issued |= 1u << st;
+                    parities = (parities & ~(1u << st)) | (ph << st);
+                }
+                else if (!kCM && tp.conv_c != 0)
                 {
                     // window origin of the tile's first output pixel; sub-blocks beyond K are not loaded at all (the
                     // MMA loop leaves them out as well)
@@ -2003,7 +2045,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         int4         *g_col   = s_col + group * BLOCK_N;
         bool          ok      = true;
         int           ti = 0;
-        int           filled_n0 = -1;
+        int           filled_nb = -1; // column block (of its product) whose terms are in g_col
         // Paired drain (see drain_accumulator_pair): the tile this group drains next (kStride ordinals on) is drained
         // together with the current one when it lies in the same column block and its accumulator buffer belongs
         // to the same phase.  The MMA warp is untouched: it fills the partner buffer while the first one waits
@@ -2013,7 +2055,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         constexpr int  kStride  = 1;
         // Two buffers only: with 128-column tiles in four buffers, pairs (0, 1) and (2, 3) drained by sixteen warps while
         // the MMA warp fills the other pair, the same layers measured slower (802816 x 256 x 64: 164 against 133 us).
-        constexpr bool kCanPair = !kCM && !kS32Out && kGroups == 1 && ACC == 2;
+        constexpr bool kCanPair = !kCM && !kS32Out && kGroups == 1 && ACC == 2 && !kBatched;
         int            skip     = -1; // ordinal of a tile already drained as the partner of an earlier one
         uint32_t       n_res_pairs = 0; // kPairTma: pairs whose residual this warp has fetched (phase of its barrier)
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++ti)
@@ -2025,19 +2067,23 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int      as  = ti % ACC;
             const uint32_t aph = static_cast<uint32_t>(ti / ACC) & 1u;
             const int      m0  = (kCM ? tile / num_n_blocks : tile % num_m_blocks) * BLOCK_M;
-            const int      n0  = (kCM ? tile % num_n_blocks : tile / num_m_blocks) * BLOCK_N;
+            const int      nb  = kCM ? tile % num_n_blocks : tile / num_m_blocks;
+            const int      z   = kBatched ? nb / num_n_blocks : -1;
+            const int      n0  = (kBatched ? nb - z * num_n_blocks : nb) * BLOCK_N;
             // The warps of a group meet only where the column terms change (tiles are ordered m-fastest, so the terms
             // usually carry over): between such points every warp waits for its accumulator, drains its share and hands
             // it back on its own, and a slow warp holds nobody up.  A warp whose wait ran out keeps walking the tile
             // list without working, so that the barrier counts stay whole until all leave together.
-            if (!kCM && n0 != filled_n0)
+            if (!kCM && nb != filled_nb)
             {
                 if (!(kGroups == 1 ? epi_barrier_and(ok) : epi_group_barrier_and(ok, group)))
                 {
                     break; // the old terms are no longer read by anyone; someone gave up
                 }
-                fill_column_terms<BLOCK_N>(g_col, et, n0, tp, ep, kEpiThreads / kGroups);
-                filled_n0 = n0;
+                EpilogueParams ec = ep;
+                if (kBatched && ec.colsum != nullptr) ec.colsum += static_cast<int64_t>(z) * tp.batch_colsum;
+                fill_column_terms<BLOCK_N>(g_col, et, n0, tp, ec, kEpiThreads / kGroups);
+                filled_nb = nb;
                 if (kGroups == 1) epi_barrier();
                 else epi_group_barrier(group);
             }
@@ -2103,9 +2149,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 else
                 {
-                    epilogue_warp_tile<BLOCK_N, kS32Out, kGroups>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane,
+                    EpilogueParams er = ep;
+                    if (kBatched && er.rowsum != nullptr) er.rowsum += static_cast<int64_t>(z) * tp.batch_rowsum;
+                    epilogue_warp_tile<BLOCK_N, kS32Out, kGroups>(tmem_base + as * BLOCK_N, g_col, tp, er, warp, lane,
                                                                   m0, n0, smem + P::OFF_OUT, rel,
-                                                                  (tp.tma_store != 0 && !kPairTma) ? &tmap_out : nullptr);
+                                                                  (tp.tma_store != 0 && !kPairTma) ? &tmap_out : nullptr, z);
                 }
                 __syncwarp();
                 if (et == 0) trace_event(tp.trace, ti, 5);
@@ -3035,18 +3083,20 @@ EncodeTiledFn get_encode_fn()
 
 // rows x K bytes, K contiguous, row stride ld; box = box_rows x 128 bytes, 128-byte swizzle; elements
 // outside [0,K) x [0,rows) read as zero, which is what makes ragged M / N / K tiles exact.
-bool encode_operand_map(CUtensorMap *map, const void *base, int rows, int K, int64_t ld, int box_rows)
+// batch > 0: a third dimension of that many matrices, batch_stride bytes apart (a multiple of 16).
+bool encode_operand_map(CUtensorMap *map, const void *base, int rows, int K, int64_t ld, int box_rows, int batch = 0,
+                        int64_t batch_stride = 0)
 {
     EncodeTiledFn fn = get_encode_fn();
     if (fn == nullptr)
     {
         return false;
     }
-    const cuuint64_t dims[2]    = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld)};
-    const cuuint32_t box[2]     = {static_cast<cuuint32_t>(BLOCK_K), static_cast<cuuint32_t>(box_rows)};
-    const cuuint32_t estr[2]    = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
+    const cuuint64_t dims[3]    = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(batch)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld), static_cast<cuuint64_t>(batch_stride)};
+    const cuuint32_t box[3]     = {static_cast<cuuint32_t>(BLOCK_K), static_cast<cuuint32_t>(box_rows), 1};
+    const cuuint32_t estr[3]    = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, batch > 0 ? 3 : 2, const_cast<void *>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -3057,19 +3107,21 @@ bool encode_operand_map(CUtensorMap *map, const void *base, int rows, int K, int
 bool encode_out_map(const GemmOperands &op, CUtensorMap *map, bool *use, int row_bytes = kOutRowBytes,
                     bool any_build = false)
 {
+    const bool batched = op.batch > 1;
     *use = (kEpiWarps <= 8 || any_build) && op.tma_store >= 0 && op.n_extra_dst == 0 &&
-           ((reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd)) & 15) == 0;
+           ((reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd) |
+             (batched ? static_cast<uint64_t>(op.d_batch_stride) : 0)) & 15) == 0;
     if (!*use)
     {
         return true;
     }
     EncodeTiledFn    fn         = get_encode_fn();
-    const cuuint64_t dims[2]    = {static_cast<cuuint64_t>(op.N), static_cast<cuuint64_t>(op.M)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(op.ldd)};
-    const cuuint32_t box[2]     = {static_cast<cuuint32_t>(row_bytes), 32};
-    const cuuint32_t estr[2]    = {1, 1};
+    const cuuint64_t dims[3]    = {static_cast<cuuint64_t>(op.N), static_cast<cuuint64_t>(op.M), static_cast<cuuint64_t>(op.batch)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(op.ldd), static_cast<cuuint64_t>(op.d_batch_stride)};
+    const cuuint32_t box[3]     = {static_cast<cuuint32_t>(row_bytes), 32, 1};
+    const cuuint32_t estr[3]    = {1, 1, 1};
     return fn != nullptr &&
-           fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, op.dst, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, batched ? 3 : 2, op.dst, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
               row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                                : (row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B),
               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -3130,43 +3182,7 @@ bool conv_tma_supported(const GemmOperands &op)
            (cv.kw - 1) * cv.dil_x < 256 && (cv.kh - 1) * cv.dil_y < 256 && get_encode_im2col_fn() != nullptr;
 }
 
-// Programmatic stream serialization pays where launches are issued one by one (QASYMM8 ResNet-50, batch 256, layer
-// by layer: 2.74 -> 2.67 ms); inside a captured graph, whose launches are packed already, the programmatic edges
-// measured 1 % slower (2.594 -> 2.618 ms), so a capturing stream gets plain launches.
-inline bool use_dependent_launch(const cugl_context *ctx)
-{
-    if (ctx->dependent_launch == 0)
-    {
-        return false;
-    }
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess)
-    {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return st == cudaStreamCaptureStatusNone;
-}
-
-// Launch with programmatic stream serialization (see griddep_wait): the kernel may start its prologue while the
-// previous kernel of the stream is finishing.  ctx->dependent_launch == 0 or a capturing stream: a plain launch.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(cugl_context *ctx, void (*kernel)(KArgs...), int grid, int threads, int smem_bytes, Args &&...args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim          = dim3(static_cast<unsigned>(grid), 1, 1);
-    cfg.blockDim         = dim3(static_cast<unsigned>(threads), 1, 1);
-    cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
-    cfg.stream           = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs    = attr;
-    cfg.numAttrs = use_dependent_launch(ctx) ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
-template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kPairTma = false>
+template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kPairTma = false, bool kBatched = false>
 cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
 {
     constexpr int ACC = BLOCK_N <= 128 ? 4 : 2; // narrow tiles: four accumulator buffers in the 512 columns
@@ -3174,8 +3190,9 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
     static_assert(P::DYN_BYTES <= 227 * 1024, "shared memory plan exceeds the sm_100 limit");
     CUtensorMap map_a, map_b;
     if (!(op.conv != nullptr ? encode_im2col_map(&map_a, *op.conv)
-                             : encode_operand_map(&map_a, op.a, op.M, op.K, op.lda, BLOCK_M)) ||
-        !encode_operand_map(&map_b, op.bt, op.N, op.K, op.ldbt, BLOCK_N))
+                             : encode_operand_map(&map_a, op.a, op.M, op.K, op.lda, BLOCK_M, kBatched ? op.batch : 0, op.a_batch_stride)) ||
+        !encode_operand_map(&map_b, op.bt, op.N, op.K, op.ldbt, BLOCK_N, kBatched ? (op.bt_batch_stride != 0 ? op.batch : 1) : 0,
+                            op.bt_batch_stride != 0 ? op.bt_batch_stride : op.ldbt * op.N))
     {
         return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncode failed for a GEMM operand");
     }
@@ -3196,7 +3213,7 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
             return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the residual tiles");
         }
     }
-    auto kernel = gemmlowp_tcgen05_kernel<BLOCK_N, STAGES, KSUB, kS32Out, false, ACC, kPairTma>;
+    auto kernel = gemmlowp_tcgen05_kernel<BLOCK_N, STAGES, KSUB, kS32Out, false, ACC, kPairTma, kBatched>;
     static bool attr_set[64] = {}; // per instantiation and device
     if (!attr_set[ctx->device & 63])
     {
@@ -3212,7 +3229,8 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
     tp.K      = op.K;
     tp.idesc  = (2u << 4) | ((op.a_signed ? 1u : 0u) << 7) | ((op.b_signed ? 1u : 0u) << 10) |
                (static_cast<uint32_t>(BLOCK_N >> 3) << 17) | (static_cast<uint32_t>(BLOCK_M >> 4) << 24);
-    tp.vec_ok = vector_flags(reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd) | extra_dst_bits(op));
+    tp.vec_ok = vector_flags(reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd) | extra_dst_bits(op) |
+                             (kBatched ? static_cast<uint64_t>(op.d_batch_stride) : 0));
     tp.status  = ctx->d_status;
     tp.tma_store = 0;
     fill_conv_params(tp, op);
@@ -3225,8 +3243,21 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
     tp.idesc_half = 0;
     tp.split_tail = 0;
     const int tiles = ((op.M + BLOCK_M - 1) / BLOCK_M) * ((op.N + BLOCK_N - 1) / BLOCK_N);
-    const int grid  = tiles < ctx->sm_count ? tiles : ctx->sm_count;
+    const long long units = static_cast<long long>(tiles) * (kBatched ? op.batch : 1);
+    if (units > INT32_MAX)
+    {
+        return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "more than 2^31 output tiles");
+    }
+    const int grid  = units < ctx->sm_count ? static_cast<int>(units) : ctx->sm_count;
     tp.tma_store = tma_store ? 1 : 0;
+    tp.batch     = kBatched ? op.batch : 1;
+    tp.batch_dst = op.d_batch_stride;
+    tp.batch_colsum = op.bt_batch_stride != 0 ? op.N : 0;
+    tp.batch_rowsum = op.M;
+    if (kBatched)
+    {
+        tp.pair_drain = 0;
+    }
     CUGL_CUDA_TRY(ctx, launch_dependent(ctx, kernel, grid, kThreads, P::DYN_BYTES, map_a, map_b, map_out, map_res, tp, ep));
     return check_cuda(ctx, cudaGetLastError(), "gemmlowp_tcgen05_kernel");
 }
@@ -3456,6 +3487,18 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
                                     bool allow_pair)
 {
     const bool s32 = ep.stage == CUGL_STAGE_NONE;
+    if (op.batch > 1)
+    {
+        // one launch over all products; only the eight-warp build holds these instantiations (gemmlowp_dispatch.cu)
+        if constexpr (kEpiWarps == 8)
+        {
+            const int bn = op.block_n > 0 ? op.block_n : (op.N > 128 ? 256 : (op.N > 64 ? 128 : 64));
+            if (bn > 128) return s32 ? launch_variant<256, 4, 1, true, false, true>(ctx, op, ep) : launch_variant<256, 4, 1, false, false, true>(ctx, op, ep);
+            if (bn > 64) return s32 ? launch_variant<128, 3, 2, true, false, true>(ctx, op, ep) : launch_variant<128, 3, 2, false, false, true>(ctx, op, ep);
+            return s32 ? launch_variant<64, 4, 2, true, false, true>(ctx, op, ep) : launch_variant<64, 4, 2, false, false, true>(ctx, op, ep);
+        }
+        return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "batched launches belong to the eight-warp build");
+    }
     // channel-major accumulators: no row-sum term (it would be a per-column quantity there) and one destination
     if (op.channel_major > 0 && ep.rowsum == nullptr && op.n_extra_dst == 0 && op.conv == nullptr)
     {

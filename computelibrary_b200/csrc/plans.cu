@@ -214,11 +214,34 @@ struct GemmCore
         return !force_simt && gemmlowp_tcgen05_supported(op);
     }
 
-    // rows x K product against B copy b_copy.
+    // B as the caller holds it ([K][ldb]); given to gemm() when the call has to re-lay it out first
+    struct RawB
+    {
+        const void *b;
+        int64_t     ldb, batch_stride;
+        int         copies;
+    };
+    // several equal products in one call: byte distances of A and dst from one to the next, B shared or one copy each
+    struct Batch
+    {
+        int     count;
+        int64_t a_stride, d_stride;
+        bool    shared_b;
+    };
+    // One launch walks a whole batch through three-dimensional tensor maps (strides up to 2^40 bytes; the descriptor's
+    // validation keeps the products apart).  The generic kernel runs product by product.
+    bool one_launch(const Batch &bt) const
+    {
+        return !force_simt && bt.a_stride < (1ll << 39) && bt.d_stride < (1ll << 39);
+    }
+
+    // rows x K product(s) against B copy b_copy (a batch with copies of its own: from b_copy on).
     cugl_status gemm(const void *d_a, int64_t lda, int rows, void *d_dst, int64_t ldd, const int32_t *d_bias,
                      int b_copy, int rowsum_off, void *const *extra_dst = nullptr, int n_extra = 0,
-                     const void *d_residual = nullptr, int res_floor = 0, int res_cap = 255)
+                     const void *d_residual = nullptr, int res_floor = 0, int res_cap = 255, const RawB *raw_b = nullptr,
+                     const Batch *batch = nullptr)
     {
+        const int n_prod = batch != nullptr ? batch->count : 1;
         GemmOperands op{};
         op.a        = d_a;
         op.bt       = d_bt + static_cast<size_t>(b_copy) * ldbt * N;
@@ -251,14 +274,36 @@ struct GemmCore
         {
             op.extra_dst[i] = extra_dst[i];
         }
-        if (!force_simt && ((reinterpret_cast<uintptr_t>(d_a) | static_cast<uint64_t>(lda)) & 15) != 0)
+        op.batch = n_prod;
+        if (n_prod > 1)
         {
-            const int64_t kp  = round_up(K, 16);
-            uint8_t      *tmp = nullptr;
-            CUGL_TRY(tmp_a_buffer(static_cast<size_t>(kp) * rows, &tmp));
-            CUGL_CUDA_TRY(ctx, cudaMemcpy2DAsync(tmp, kp, d_a, lda, K, rows, cudaMemcpyDeviceToDevice, ctx->stream));
-            op.a   = tmp; // bytes K .. kp-1 of a row are never read: the tensor map ends at K
-            op.lda = kp;
+            op.a_batch_stride  = batch->a_stride;
+            op.d_batch_stride  = batch->d_stride;
+            op.bt_batch_stride = batch->shared_b ? 0 : ldbt * N;
+        }
+        // Everything that has to happen to the operands first goes into one launch: the K-major copy of a B that changes
+        // with the call, the row sums, and rows of 16-byte pitch where the TMA engine cannot address A itself.
+        OperandPrep prep{};
+        prep.N = N, prep.K = K;
+        if (raw_b != nullptr)
+        {
+            prep.b = static_cast<const uint8_t *>(raw_b->b), prep.ldb = raw_b->ldb, prep.b_batch_stride = raw_b->batch_stride;
+            prep.bt = d_bt, prep.ldbt = ldbt, prep.colsum = d_colsum, prep.b_signed = b_signed, prep.batch_b = raw_b->copies;
+        }
+        const bool unaligned = !force_simt && ((reinterpret_cast<uintptr_t>(d_a) | static_cast<uint64_t>(lda) |
+                                                (n_prod > 1 ? static_cast<uint64_t>(batch->a_stride) : 0)) & 15) != 0;
+        if (unaligned || b_off != 0)
+        {
+            prep.a = static_cast<const uint8_t *>(d_a), prep.lda = lda, prep.rows = rows, prep.batch_a = n_prod, prep.a_signed = a_signed;
+            prep.a_batch_stride = n_prod > 1 ? batch->a_stride : 0;
+        }
+        if (unaligned)
+        {
+            prep.kp = round_up(K, 16);
+            CUGL_TRY(tmp_a_buffer(static_cast<size_t>(prep.kp) * rows * n_prod, &prep.copy));
+            op.a              = prep.copy;
+            op.lda            = prep.kp;
+            op.a_batch_stride = n_prod > 1 ? prep.kp * rows : 0;
         }
         if ((n_extra > 0 || d_residual != nullptr) && !uses_tcgen05(op))
         {
@@ -271,9 +316,17 @@ struct GemmCore
         {
             CUGL_TRY(rowsum_buffer(&rowsum));
             rowsum += rowsum_off;
-            CUGL_TRY(launch_reduce_rows(ctx, op.a, a_signed, rows, K, op.lda, 1, rowsum));
+            prep.rowsum = rowsum;
+        }
+        if (prep.a != nullptr || prep.b != nullptr)
+        {
+            CUGL_TRY(launch_prepare_operands(ctx, prep));
         }
         const EpilogueParams ep = epilogue(d_bias, b_copy, rowsum);
+        if (n_prod > 1 && !uses_tcgen05(op))
+        {
+            return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled is not available");
+        }
         return uses_tcgen05(op) ? launch_gemmlowp_tcgen05(ctx, op, ep, allow_pair) : launch_gemmlowp_simt(ctx, op, ep);
     }
 };
@@ -395,14 +448,8 @@ void apply_quant_fields(cugl_gemm_plan *p, const cugl_gemm_desc *d)
 cugl_status relayout_b(cugl_gemm_plan *p, const void *d_b)
 {
     const cugl_gemm_desc &d = p->desc;
-    for (int i = 0; i < p->b_copies; ++i)
-    {
-        const uint8_t *src = static_cast<const uint8_t *>(d_b) + static_cast<int64_t>(i) * d.b_batch_stride;
-        CUGL_TRY(launch_transpose_colsum(p->ctx, src, p->core.b_signed, d.K, d.N, d.ldb,
-                                         p->core.d_bt + static_cast<size_t>(i) * p->core.ldbt * d.N, p->core.ldbt,
-                                         p->core.d_colsum + static_cast<size_t>(i) * d.N));
-    }
-    return CUGL_SUCCESS;
+    return launch_transpose_colsum(p->ctx, d_b, p->core.b_signed, d.K, d.N, d.ldb, p->core.d_bt, p->core.ldbt, p->core.d_colsum,
+                                   p->b_copies, d.b_batch_stride);
 }
 } // namespace
 
@@ -460,7 +507,7 @@ extern "C"
         c.dst_dtype = desc->dst_dtype;
         apply_quant_fields(p, desc);
         c.lda_hint   = desc->lda;
-        c.tmp_a_rows = p->collapse_batch ? desc->M * desc->batch : desc->M;
+        c.tmp_a_rows = desc->M * desc->batch; // a batch is copied in one go
         cugl_status s = c.alloc(p->b_copies, desc->M * desc->batch);
         if (s == CUGL_SUCCESS)
         {
@@ -516,20 +563,27 @@ extern "C"
         {
             return fail(plan->ctx, CUGL_INVALID_ARGUMENT, "cugl_gemmlowp_run: plan was configured with a bias");
         }
-        if (!plan->prepared || !d.reshape_b_only_on_first_run)
+        const bool new_b = !plan->prepared || !d.reshape_b_only_on_first_run;
+        if (new_b && d_b == nullptr)
         {
-            if (d_b == nullptr)
-            {
-                return fail(plan->ctx, CUGL_INVALID_ARGUMENT,
-                            "cugl_gemmlowp_run: B is required (not prepared, or B is not constant)");
-            }
+            return fail(plan->ctx, CUGL_INVALID_ARGUMENT,
+                        "cugl_gemmlowp_run: B is required (not prepared, or B is not constant)");
+        }
+        const GemmCore::RawB  raw{d_b, d.ldb, d.b_batch_stride, plan->b_copies};
+        const GemmCore::Batch all{d.batch, d.a_batch_stride, d.d_batch_stride, plan->b_copies == 1};
+        const int32_t        *bias = d.has_bias ? d_bias : nullptr;
+        if (plan->collapse_batch || d.batch == 1 || plan->core.one_launch(all))
+        {
+            const bool one = plan->collapse_batch || d.batch == 1;
+            CUGL_TRY(plan->core.gemm(d_a, d.lda, one ? d.M * d.batch : d.M, d_dst, d.ldd, bias, 0, 0, nullptr, 0, nullptr, 0, 255,
+                                     new_b ? &raw : nullptr, one ? nullptr : &all));
+            plan->prepared = true;
+            return CUGL_SUCCESS;
+        }
+        if (new_b)
+        {
             CUGL_TRY(relayout_b(plan, d_b));
             plan->prepared = true;
-        }
-        const int32_t *bias = d.has_bias ? d_bias : nullptr;
-        if (plan->collapse_batch || d.batch == 1)
-        {
-            return plan->core.gemm(d_a, d.lda, d.M * d.batch, d_dst, d.ldd, bias, 0, 0);
         }
         for (int i = 0; i < d.batch; ++i)
         {
@@ -824,13 +878,12 @@ extern "C"
             return 0;
         }
         const cugl_gemm_desc &d       = plan->desc;
-        const int             n_gemms = (plan->collapse_batch || d.batch == 1) ? 1 : d.batch;
-        int                   n       = n_gemms * (1 + (plan->core.b_off != 0 ? 1 : 0));
-        if (!d.reshape_b_only_on_first_run)
-        {
-            n += plan->b_copies;
-        }
-        return n;
+        const GemmCore       &c = plan->core;
+        const GemmCore::Batch all{d.batch, d.a_batch_stride, d.d_batch_stride, plan->b_copies == 1};
+        const bool one   = plan->collapse_batch || d.batch == 1 || c.one_launch(all);
+        const bool rows  = c.b_off != 0 || (!c.force_simt && (d.lda & 15) != 0); // the operand preparation looks at A
+        const bool new_b = !d.reshape_b_only_on_first_run;
+        return one ? 1 + (rows || new_b ? 1 : 0) : d.batch * (rows ? 2 : 1) + (new_b ? 1 : 0);
     }
 
     // ---- stand-alone kernels ---------------------------------------------------------------------

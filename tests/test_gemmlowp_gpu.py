@@ -139,6 +139,41 @@ def test_batched(ctx, port):
         assert np.array_equal(acc, port.gemmlowp_core(a, b, 4, -6))
 
 
+@pytest.mark.parametrize("batch,M,N,K,ldd_pad", [(2, 1, 1, 1, 0), (3, 129, 65, 17, 0), (5, 128, 256, 128, 16), (4, 300, 257, 259, 3),
+                                                 (7, 31, 593, 23, 0), (2, 257, 130, 1100, 14), (3, 64, 48, 4224, 0), (40, 130, 16, 33, 0)])
+def test_batch_in_one_launch(ctx, port, batch, M, N, K, ldd_pad):
+    """Products of a batch walked by one launch: tile edges and remainders in every direction, aligned and unaligned rows
+    of A, B and dst (canary bytes between and around the products), own and shared B, B that changes with the call."""
+    rng = np.random.default_rng(batch * 1000 + K)
+    for t, signed in ((np.uint8, False), (np.int8, True)):
+        a, b3 = q8_uniform(rng, (batch, M, K), t), q8_uniform(rng, (batch, K, N), t)
+        a_off, b_off = (3, -5) if signed else (-128, -120)
+        qm, sh = capi.calculate_quantized_multiplier(np.float32(0.5 / (73 * np.sqrt(K))))
+        lo, hi = type_range(t)
+        bias = rng.integers(-2000, 2001, N).astype(np.int32)
+        for b, const in ((b3, False), (b3, True), (b3[0], True)):
+            got, kernel = gpu_gemmlowp(ctx, a, b, bias, a_off, b_off, qm, sh, 7, lo, hi, t, b_constant=const, ldd_pad=ldd_pad, runs=2,
+                                       temp_workspace=const)
+            assert kernel.startswith("tcgen05")
+            for i in range(batch):
+                want = port.gemmlowp_fused(a[i], b if b.ndim == 2 else b[i], bias, a_off, b_off, [qm], [sh], 7, lo, hi, t)
+                assert np.array_equal(got[i], want), (t, const, b.ndim, i)
+        acc, _ = gpu_gemmlowp(ctx, a, b3, None, a_off, 0, 0, 0, 0, 0, 0, np.int32, b_constant=False, ldd_pad=ldd_pad)
+        assert np.array_equal(acc, port.gemmlowp_core(a, b3, a_off, 0))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (5, 63, 19), (129, 65, 130), (40, 4, 127), (33, 1000, 513), (200, 96, 3000)])
+def test_operand_preparation(ctx, port, M, N, K):
+    """Row sums, realigned rows of A and the K-major copy of B with its column sums, over remainders of every tile edge;
+    K ranges one block walks alone and ranges split over blocks."""
+    rng = np.random.default_rng(M + K)
+    for ta, tb in ((np.uint8, np.uint8), (np.int8, np.int8), (np.uint8, np.int8)):
+        a, b = q8_uniform(rng, (M, K), ta), q8_uniform(rng, (K, N), tb)
+        for const in (True, False):
+            acc, _ = gpu_gemmlowp(ctx, a, b, None, 11, -7, 0, 0, 0, 0, 0, np.int32, b_constant=const, runs=2)
+            assert np.array_equal(acc, port.gemmlowp_core(a, b, 11, -7))
+
+
 def test_run_twice_and_variable_b(ctx, port):
     """MultipleExecution (GEMMLowp.cpp:211-297): same plan, same output; B re-laid out per run when it is
     not constant (reshape_b_only_on_first_run = false)."""
