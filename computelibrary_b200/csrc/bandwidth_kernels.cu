@@ -545,6 +545,20 @@ struct Im2colDivs
     FastDiv units, c, kw, wo, ho;
 };
 
+// weights of a convolution whose channels are padded (once per weight tensor): [rows][taps][C] -> [rows][taps][Cp]
+__global__ void __launch_bounds__(kThreads) spread_channels_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
+                                                                   int rows, int taps, int C, int Cp, int64_t ldd)
+{
+    const int64_t total = static_cast<int64_t>(rows) * taps * Cp;
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(kThreads) + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * kThreads)
+    {
+        const int64_t t = i / Cp; // (row, tap)
+        const int     c = static_cast<int>(i - t * Cp);
+        const int64_t r = t / taps;
+        dst[r * ldd + (t - r * taps) * Cp + c] = c < C ? src[t * C + c] : 0;
+    }
+}
+
 template <int VEC>
 __global__ void __launch_bounds__(kThreads) im2col_nhwc_kernel(const uint8_t *__restrict__ src,
                                                                uint8_t *__restrict__ dst, int C, int W, int H,
@@ -863,6 +877,14 @@ cugl_status launch_output_stage(cugl_context *ctx, const int32_t *d_in, int64_t 
             shift, offset, lo, hi, vec_ok, integer_stage);
     }
     return check_cuda(ctx, cudaGetLastError(), "output_stage_kernel");
+}
+
+cugl_status launch_spread_channels(cugl_context *ctx, const void *d_src, void *d_dst, int rows, int taps, int C, int Cp, int64_t ldd)
+{
+    const int blocks = grid_for(static_cast<int64_t>(rows) * taps * Cp, ctx->sm_count);
+    spread_channels_kernel<<<blocks, kThreads, 0, ctx->stream>>>(static_cast<const uint8_t *>(d_src), static_cast<uint8_t *>(d_dst), rows,
+                                                                 taps, C, Cp, ldd);
+    return check_cuda(ctx, cudaGetLastError(), "spread_channels_kernel");
 }
 
 cugl_status launch_im2col_nhwc(cugl_context *ctx, const void *d_src, void *d_dst, int C, int W, int H, int B, int kw,

@@ -1620,18 +1620,21 @@ __device__ __forceinline__ void epilogue_warp_tile_cm(uint32_t tmem_acc, const T
 // The part of a tile one epilogue warp owns: lane quarter (warp & 3) and half of the columns.
 // kGroups = 2: the eight epilogue warps form two groups of four that drain alternate tiles, each warp all columns
 // of its 32 rows (narrow tiles, whose time is latency rather than work).
-template <int BLOCK_N, bool kS32Out, int kGroups = 1>
+// kGivenRowTerm: the caller has worked out the row term itself (window sums of a convolution)
+template <int BLOCK_N, bool kS32Out, int kGroups = 1, bool kGivenRowTerm = false>
 __device__ __forceinline__ void epilogue_warp_tile(uint32_t tmem_acc, const int4 *s_col, const TileParams &tp,
                                                    const EpilogueParams &ep, int warp, int lane, int m0, int n0,
                                                    uint8_t *out_stage, const AccRelease &rel,
-                                                   const CUtensorMap *omap = nullptr, int z = -1)
+                                                   const CUtensorMap *omap = nullptr, int z = -1,
+                                                   int32_t given_row_term = 0)
 {
     constexpr int NCOLS    = BLOCK_N * kGroups / (kEpiWarps / 4);
     uint8_t      *stage    = out_stage + (warp - kFirstEpi) * kOutStageBytes;
     const int     quad     = warp & 3;               // tensor-memory lane quarter this warp may read
     const int     half     = kGroups == 1 ? (warp - kFirstEpi) >> 2 : 0; // which share of the columns
     const int     m        = m0 + quad * 32 + lane;
-    const int32_t row_term = (ep.rowsum != nullptr && m < tp.M) ? ep.b_off * __ldg(ep.rowsum + m) : 0;
+    const int32_t row_term =
+        kGivenRowTerm ? given_row_term : ((ep.rowsum != nullptr && m < tp.M) ? ep.b_off * __ldg(ep.rowsum + m) : 0);
     const uint32_t t_addr  = tmem_acc + (static_cast<uint32_t>(quad * 32) << 16) + half * NCOLS;
     if (tp.mode == kStagePack && !kS32Out)
     {
@@ -2080,9 +2083,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 {
                     break; // the old terms are no longer read by anyone; someone gave up
                 }
-                EpilogueParams ec = ep;
-                if (kBatched && ec.colsum != nullptr) ec.colsum += static_cast<int64_t>(z) * tp.batch_colsum;
-                fill_column_terms<BLOCK_N>(g_col, et, n0, tp, ec, kEpiThreads / kGroups);
+                if constexpr (kBatched)
+                {
+                    EpilogueParams ec = ep;
+                    if (ec.colsum != nullptr) ec.colsum += static_cast<int64_t>(z) * tp.batch_colsum;
+                    fill_column_terms<BLOCK_N>(g_col, et, n0, tp, ec, kEpiThreads / kGroups);
+                }
+                else
+                {
+                    fill_column_terms<BLOCK_N>(g_col, et, n0, tp, ep, kEpiThreads / kGroups);
+                }
                 filled_nb = nb;
                 if (kGroups == 1) epi_barrier();
                 else epi_group_barrier(group);
@@ -2149,11 +2159,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 else
                 {
-                    EpilogueParams er = ep;
-                    if (kBatched && er.rowsum != nullptr) er.rowsum += static_cast<int64_t>(z) * tp.batch_rowsum;
-                    epilogue_warp_tile<BLOCK_N, kS32Out, kGroups>(tmem_base + as * BLOCK_N, g_col, tp, er, warp, lane,
-                                                                  m0, n0, smem + P::OFF_OUT, rel,
-                                                                  (tp.tma_store != 0 && !kPairTma) ? &tmap_out : nullptr, z);
+                    const CUtensorMap *omap = (tp.tma_store != 0 && !kPairTma) ? &tmap_out : nullptr;
+                    if constexpr (kBatched)
+                    {
+                        EpilogueParams er = ep;
+                        if (er.rowsum != nullptr) er.rowsum += static_cast<int64_t>(z) * tp.batch_rowsum;
+                        epilogue_warp_tile<BLOCK_N, kS32Out, kGroups>(tmem_base + as * BLOCK_N, g_col, tp, er, warp, lane, m0, n0,
+                                                                      smem + P::OFF_OUT, rel, omap, z);
+                    }
+                    else
+                    {
+                        epilogue_warp_tile<BLOCK_N, kS32Out, kGroups>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane, m0, n0,
+                                                                      smem + P::OFF_OUT, rel, omap);
+                    }
                 }
                 __syncwarp();
                 if (et == 0) trace_event(tp.trace, ti, 5);
@@ -2588,7 +2606,39 @@ struct ConvGeom
     const uint8_t *pad; // 16 bytes of the input zero point per gather thread (kConvPadBytes in all)
     int            C, W, H, kw, kh, sx, sy, pad_l, pad_t, dil_x, dil_y, Wo, Ho;
     FastDiv        div_wo, div_ho;
+    int32_t        pad_sum; // channel sum of an out-of-image tap (asymmetric weights)
 };
+
+// Asymmetric weights: sum over the patch of output pixel m, from the channel sums of the input pixels.  A kh x kw window
+// of sums is C times less to read than the patch itself, and the epilogue warps read it while they would otherwise wait
+// for the accumulators.  A call of its own: inlined, it costs the symmetric case registers (96 per thread, spills).
+__device__ __noinline__ int32_t window_sum(const int32_t *__restrict__ pixel_sums, int m, const ConvGeom &cg)
+{
+    const int q  = fast_div(m, cg.div_wo), xo = m - q * cg.Wo;
+    const int bi = fast_div(q, cg.div_ho), yo = q - bi * cg.Ho;
+    const int y0 = yo * cg.sy - cg.pad_t, x0 = xo * cg.sx - cg.pad_l;
+    const int32_t *image = pixel_sums + static_cast<int64_t>(bi) * cg.H * cg.W;
+    int32_t        sum   = 0;
+    int            x = x0, y = y0, kx = 0;
+    for (int left = cg.kh * cg.kw; left > 0; left -= 9) // nine loads in flight: a 3 x 3 window at once
+    {
+        int32_t v[9];
+#pragma unroll
+        for (int j = 0; j < 9; ++j)
+        {
+            const bool in = static_cast<unsigned>(y) < static_cast<unsigned>(cg.H) && static_cast<unsigned>(x) < static_cast<unsigned>(cg.W);
+            v[j]          = j >= left ? 0 : (in ? __ldg(image + static_cast<int64_t>(y) * cg.W + x) : cg.pad_sum);
+            x += cg.dil_x;
+            if (++kx == cg.kw)
+            {
+                kx = 0, x = x0, y += cg.dil_y;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 9; ++j) sum += v[j];
+    }
+    return sum;
+}
 
 // One entry per 16-byte piece of the patch axis: where the piece lies relative to the top-left tap of an
 // output pixel.  Built once per CTA in shared memory so that the gather loop has no division in it.
@@ -2597,7 +2647,7 @@ struct TapEntry
     int32_t  offset; // bytes from the (ky = 0, kx = 0, c = 0) element, in the input tensor
     uint32_t dydx;   // (ky * dilation_y) << 16 | (kx * dilation_x)
 };
-constexpr int kConvMaxPieces = 1024; // K <= 16384 bytes
+constexpr int kConvMaxPieces = kConvMaxK / 16;
 
 constexpr int kGatherWarps  = 8;
 static_assert(kConvPadBytes >= 16 * 32 * kGatherWarps, "one pad piece per gather thread");
@@ -2614,7 +2664,8 @@ constexpr int kConvThreads  = kThreads + 32 * kGatherWarps;
 template <int BLOCK_N, int STAGES, int KSUB, int ACC, int RESB = 0, int MT = 1>
 __global__ void __launch_bounds__(kConvThreads, 1)
     gemmlowp_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_out,
-                                 const __grid_constant__ TileParams tp, const EpilogueParams ep, const ConvGeom cg)
+                                 const __grid_constant__ TileParams tp, const EpilogueParams ep,
+                                 const __grid_constant__ ConvGeom cg)
 {
     using P = SmemPlan<BLOCK_N, STAGES, MT * KSUB, ACC, false, RESB>; // the A ring: MT x KSUB sub-tiles per stage
     static_assert(MT == 1 || (MT == 2 && RESB != 0 && ACC == 4 && P::EPI_GROUPS == 2), "double tiles: resident B, four buffers, two groups");
@@ -2878,14 +2929,17 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 if (kGroups == 1) epi_barrier();
                 else epi_group_barrier(group);
             }
+            const int      m_row    = m0 + (warp & 3) * 32 + lane;
+            const int32_t  row_term = (ep.rowsum != nullptr && m_row < tp.M) ? ep.b_off * window_sum(ep.rowsum, m_row, cg) : 0;
             ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(as_first), aph, s_abort, DEV_TIMEOUT_EPILOGUE, tp.spin_limit));
             if (ok)
             {
                 tc_fence_after();
                 if (et == 0) trace_event(tp.trace, ti, 4);
                 const AccRelease rel{tempty_bar(as), 0u, false};
-                epilogue_warp_tile<BLOCK_N, false, kGroups>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane, m0, n0,
-                                                            smem + P::OFF_OUT, rel, tp.tma_store != 0 ? &tmap_out : nullptr);
+                epilogue_warp_tile<BLOCK_N, false, kGroups, true>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane, m0, n0,
+                                                                  smem + P::OFF_OUT, rel, tp.tma_store != 0 ? &tmap_out : nullptr,
+                                                                  -1, row_term);
                 if (et == 0) trace_event(tp.trace, ti, 5);
                 __syncwarp();
             }
@@ -3446,6 +3500,7 @@ cugl_status launch_conv_variant(cugl_context *ctx, const GemmOperands &op, const
     cg.Ho    = cv.Ho;
     cg.div_wo = make_fastdiv(cv.Wo);
     cg.div_ho = make_fastdiv(cv.Ho);
+    cg.pad_sum = cv.pad_sum;
     const int tiles = ((op.M + MT * BLOCK_M - 1) / (MT * BLOCK_M)) * ((op.N + BLOCK_N - 1) / BLOCK_N); // units of MT tiles
     const int grid  = tiles < ctx->sm_count ? tiles : ctx->sm_count;
     tp.tma_store = tma_store ? 1 : 0;

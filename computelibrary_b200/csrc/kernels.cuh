@@ -48,6 +48,8 @@ cugl_status launch_fold_input(cugl_context *ctx, const void *d_src, void *d_dst,
                               int W2, int zero_point);
 cugl_status launch_fold_weights(cugl_context *ctx, const void *d_w, void *d_bt, int64_t ldbt, int OFM, int kh, int kw,
                                 int C, int kh2, int kw2, int oy, int ox);
+// [rows][taps][C] bytes -> [rows][taps][Cp], Cp >= C (zeros behind C), rows of dst ldd bytes apart
+cugl_status launch_spread_channels(cugl_context *ctx, const void *d_src, void *d_dst, int rows, int taps, int C, int Cp, int64_t ldd);
 cugl_status launch_im2col_nhwc(cugl_context *ctx, const void *d_src, void *d_dst, int C, int W, int H, int B, int kw,
                                int kh, int sx, int sy, int pad_l, int pad_t, int dil_x, int dil_y, int Wo, int Ho,
                                int pad_value, int64_t row_stride);
@@ -109,11 +111,15 @@ struct GemmOperands
 // Geometry of an NHWC 8-bit convolution whose A operand is gathered on the fly (implicit GEMM).
 // bytes of the zero-point pad buffer of the implicit convolution: 16 per gather thread
 constexpr int kConvPadBytes = 16 * 256;
+constexpr int kConvMaxK     = 16384; // patch bytes the implicit kernel's tap table holds
 
 struct ConvOperands
 {
     const void    *src;    // [B][H][W][C]
     const void    *pad;    // kConvPadBytes holding the input zero point (source of out-of-image taps)
+    // asymmetric weights: EpilogueParams::rowsum holds the channel sum of every input PIXEL, the kernel adds up the window
+    // of each output pixel; pad_sum is the channel sum of an out-of-image tap
+    int32_t        pad_sum;
     int            C, W, H, B, kw, kh, sx, sy, pad_l, pad_t, dil_x, dil_y, Wo, Ho;
 };
 bool        gemmlowp_conv_tcgen05_supported(const GemmOperands &op, const ConvOperands &cv);

@@ -49,6 +49,7 @@ struct GemmCore
     uint8_t      *d_tmp_a_bound = nullptr; // inside the caller's temporary workspace
     int64_t       lda_hint = 0;            // row pitch of A announced at configure time (sizes the workspace share)
     int           tmp_a_rows = 0;          // rows one launch copies at most
+    size_t        tmp_a_need = 0;          // > 0: the copy needs this many bytes whatever lda_hint says (convolution inputs)
     int32_t      *d_mults  = nullptr; // [N]
     int32_t      *d_shifts = nullptr;
     bool          force_simt = false;
@@ -74,6 +75,7 @@ struct GemmCore
 
     size_t tmp_a_bytes() const
     {
+        if (tmp_a_need != 0) return static_cast<size_t>(round_up(static_cast<int64_t>(tmp_a_need), 256));
         return (lda_hint & 15) != 0 ? static_cast<size_t>(round_up(round_up(K, 16) * static_cast<int64_t>(tmp_a_rows), 256)) : 0;
     }
 
@@ -1029,6 +1031,10 @@ struct cugl_conv_plan
     bool     fold = false;
     int      eC = 0, eW = 0, eH = 0, ekw = 0, ekh = 0, esx = 1, esy = 1, epl = 0, ept = 0;
     int      fold_oy = 0, fold_ox = 0;
+    // Channels that are not a multiple of 16: the input is copied with every pixel padded to eC channels of the input zero
+    // point, the weights with zero weights there.  Such a channel contributes (zp - zp) * (0 - w_zp) = 0, so the padded
+    // problem is the same convolution and every lowering works on it unchanged.
+    bool     pad_c = false;
     uint8_t *d_fold = nullptr; // [B][eH][eW][16]; plan-owned, allocated on first use unless a workspace is bound
     // temporary workspace handed in by the caller (cugl_conv2d_plan_bind_temp): row sums | folded input | im2col matrix
     uint8_t *d_temp = nullptr;
@@ -1048,7 +1054,11 @@ struct cugl_conv_plan
     }
     size_t temp_bytes() const
     {
-        return core.rowsum_bytes() + fold_bytes() + cols_bytes();
+        return core.rowsum_bytes() + fold_bytes() + core.tmp_a_bytes() + cols_bytes();
+    }
+    int64_t pixels() const // of the input the lowerings see
+    {
+        return static_cast<int64_t>(desc.B) * eH * eW;
     }
     // fused residual addition (cugl_conv2d_plan_set_residual): clamp bounds of the saturating form
     bool residual_set = false;
@@ -1160,14 +1170,20 @@ extern "C"
             p->esx = p->esy = 1;
             p->epl = (desc->pad_left + p->fold_ox) / 2, p->ept = (desc->pad_top + p->fold_oy) / 2;
         }
+        const bool pointwise = desc->kw == 1 && desc->kh == 1 && desc->stride_x == 1 && desc->stride_y == 1 && desc->pad_left == 0 &&
+                               desc->pad_right == 0 && desc->pad_top == 0 && desc->pad_bottom == 0;
+        const bool countable = static_cast<int64_t>(desc->B) * desc->H * desc->W <= INT32_MAX; // pixels as 32-bit rows
+        p->pad_c = !p->fold && !pointwise && (desc->C % 16) != 0 && countable;
+        if (p->pad_c)
+        {
+            p->eC = static_cast<int>(round_up(desc->C, 16));
+        }
         p->M  = static_cast<int64_t>(desc->B) * p->Ho * p->Wo;
         p->K  = static_cast<int64_t>(p->ekh) * p->ekw * p->eC;
         p->Kp = round_up(p->K, 16);
         // CpuGemmConv2d.cpp:189-191: a 1x1, stride-1, unpadded NHWC convolution is a plain GEMM on the
-        // input tensor.  Kept only when the rows are already 16-byte multiples (TMA stride rule).
-        p->skip_im2col = desc->kw == 1 && desc->kh == 1 && desc->stride_x == 1 && desc->stride_y == 1 &&
-                         desc->pad_left == 0 && desc->pad_right == 0 && desc->pad_top == 0 &&
-                         desc->pad_bottom == 0 && (desc->C % 16) == 0;
+        // input tensor; rows that are not 16-byte multiples are copied first (GemmCore::gemm).
+        p->skip_im2col = pointwise;
         GemmCore &c     = p->core;
         c.ctx           = ctx;
         c.M             = static_cast<int>(p->M);
@@ -1185,14 +1201,19 @@ extern "C"
         c.result_offset = desc->dst_zero_point;
         c.min_bound     = desc->min_bound;
         c.max_bound     = desc->max_bound;
-        cugl_status s   = c.alloc(1, c.M);
+        const int64_t staged_rows = p->pad_c ? p->pixels() : (p->skip_im2col && (desc->C % 16) != 0 ? p->M : 0);
+        c.tmp_a_need              = static_cast<size_t>(staged_rows) * static_cast<size_t>(round_up(desc->C, 16));
+        // Implicit GEMM whenever the gather kernel can address the tensors: 16-byte channel pieces (padded if need be) and the
+        // limits of its tap table (gemmlowp_conv_tcgen05_supported).  Otherwise explicit im2col.
+        p->implicit = !p->skip_im2col && (p->eC % 16) == 0 && p->K <= kConvMaxK &&
+                      static_cast<int64_t>(p->eH) * p->eW * p->eC < (1ll << 31) && (desc->w_zero_point == 0 || countable);
+        // row sums: one per output pixel, or (implicit kernel) one channel sum per input pixel
+        const int64_t n_sums = p->implicit && countable && p->pixels() > p->M ? p->pixels() : p->M;
+        cugl_status   s      = c.alloc(1, static_cast<int>(n_sums));
         if (s == CUGL_SUCCESS)
         {
             s = c.upload_stage_vectors(p->h_mults.data(), p->h_shifts.data());
         }
-        // Implicit GEMM whenever the gather kernel can address the tensors: channel count a multiple of 16 and
-        // symmetric weights (no row-sum term).  Otherwise explicit im2col.
-        p->implicit = !p->skip_im2col && (p->eC % 16) == 0 && desc->w_zero_point == 0;
         if (s == CUGL_SUCCESS && p->implicit)
         {
             s = cugl_malloc(ctx, kConvPadBytes, reinterpret_cast<void **>(&p->d_pad));
@@ -1243,6 +1264,10 @@ extern "C"
             const cugl_conv_desc &d = plan->desc;
             CUGL_TRY(launch_fold_weights(ctx, d_weights, c.d_bt, c.ldbt, c.N, d.kh, d.kw, d.C, plan->ekh, plan->ekw,
                                          plan->fold_oy, plan->fold_ox));
+        }
+        else if (plan->pad_c)
+        {
+            CUGL_TRY(launch_spread_channels(ctx, d_weights, c.d_bt, c.N, plan->ekh * plan->ekw, plan->desc.C, plan->eC, c.ldbt));
         }
         else
         {
@@ -1342,7 +1367,30 @@ extern "C"
                                        d.src_zero_point));
             d_src = fold_buf;
         }
-        if (plan->implicit && plan->allow_implicit && !plan->core.force_simt)
+        const bool implicit_now = plan->implicit && plan->allow_implicit && !plan->core.force_simt;
+        int32_t   *pixel_sums   = nullptr;
+        if (plan->pad_c || (implicit_now && plan->core.b_off != 0))
+        {
+            // one pass over the input: the copy with padded channels and / or the channel sum of every pixel
+            GemmCore   &c = plan->core;
+            OperandPrep prep{};
+            prep.a = static_cast<const uint8_t *>(d_src), prep.lda = d.C, prep.batch_a = 1, prep.a_signed = c.a_signed;
+            prep.rows = static_cast<int>(plan->pixels()), prep.K = d.C;
+            if (plan->pad_c)
+            {
+                prep.kp   = plan->eC;
+                prep.fill = d.src_zero_point & 0xff;
+                CUGL_TRY(c.tmp_a_buffer(c.tmp_a_need, &prep.copy));
+            }
+            if (implicit_now && c.b_off != 0)
+            {
+                CUGL_TRY(c.rowsum_buffer(&pixel_sums));
+                prep.rowsum = pixel_sums;
+            }
+            CUGL_TRY(launch_prepare_operands(plan->ctx, prep));
+            if (plan->pad_c) d_src = prep.copy;
+        }
+        if (implicit_now)
         {
             GemmCore    &c = plan->core;
             GemmOperands op{};
@@ -1389,10 +1437,13 @@ extern "C"
             cv.dil_y  = d.dil_y;
             cv.Wo     = plan->Wo;
             cv.Ho     = plan->Ho;
+            const int zp_byte = d.src_zero_point & 0xff;
+            cv.pad_sum        = plan->eC * (c.a_signed ? static_cast<int8_t>(zp_byte) : zp_byte);
             // Input zero point 0 and whole 128-channel blocks: the TMA unit builds the patch tiles itself (im2col-mode
             // tensor map, out-of-image taps read as zero = the zero point) and the GEMM kernels run unchanged; else
             // the gather kernel, whose out-of-image taps copy any zero point from the pad buffer.
-            if (plan->allow_tma_im2col != 0 && d.src_zero_point == 0 && (plan->eC != 64 || plan->allow_tma_im2col > 1))
+            // (symmetric weights only: the window sums of asymmetric ones are the gather kernel's)
+            if (plan->allow_tma_im2col != 0 && d.src_zero_point == 0 && c.b_off == 0 && (plan->eC != 64 || plan->allow_tma_im2col > 1))
             {
                 GemmOperands ot  = op;
                 ot.conv          = &cv;
@@ -1404,14 +1455,17 @@ extern "C"
             }
             if (gemmlowp_conv_tcgen05_supported(op, cv))
             {
-                return launch_gemmlowp_conv_tcgen05(plan->ctx, op, c.epilogue(d.has_bias ? d_bias : nullptr, 0), cv);
+                return launch_gemmlowp_conv_tcgen05(plan->ctx, op, c.epilogue(d.has_bias ? d_bias : nullptr, 0, pixel_sums), cv);
             }
         }
         const void *a   = d_src;
         int64_t     lda = plan->eC;
         if (!plan->skip_im2col)
         {
-            uint8_t *cols = bound ? plan->d_temp + plan->core.rowsum_bytes() + plan->fold_bytes() : plan->d_cols;
+            // (a plan of the implicit kernel comes here only for a source it cannot address, which no workspace provides for)
+            uint8_t *cols = bound && plan->cols_bytes() != 0
+                                ? plan->d_temp + plan->core.rowsum_bytes() + plan->fold_bytes() + plan->core.tmp_a_bytes()
+                                : plan->d_cols;
             if (cols == nullptr)
             {
                 CUGL_TRY(cugl_malloc(plan->ctx, static_cast<size_t>(plan->M) * plan->Kp,
@@ -1574,7 +1628,7 @@ extern "C"
     {
         // the conditions the plan can see; the run adds the alignment of the source pointer (16 bytes)
         return plan != nullptr && plan->implicit && plan->allow_implicit && !plan->core.force_simt && plan->allow_tma_im2col != 0 &&
-                       plan->desc.src_zero_point == 0 && ((plan->eC % 128) == 0 || (plan->eC == 64 && plan->allow_tma_im2col > 1))
+                       plan->desc.src_zero_point == 0 && plan->core.b_off == 0 && ((plan->eC % 128) == 0 || (plan->eC == 64 && plan->allow_tma_im2col > 1))
                    ? 1
                    : 0;
     }
@@ -1601,9 +1655,10 @@ extern "C"
         const int fold = plan->fold ? 1 : 0;
         if (plan->implicit && plan->allow_implicit)
         {
-            return fold + 1;
+            return fold + (plan->pad_c || plan->core.b_off != 0 ? 1 : 0) + 1;
         }
-        return fold + (plan->skip_im2col ? 0 : 1) + 1 + (plan->core.b_off != 0 ? 1 : 0);
+        const bool rows = plan->core.b_off != 0 || (plan->skip_im2col && (plan->desc.C & 15) != 0);
+        return fold + (plan->pad_c ? 1 : 0) + (plan->skip_im2col ? 0 : 1) + 1 + (rows ? 1 : 0);
     }
     cugl_status cugl_conv2d_update_quantization(cugl_conv_plan *plan, const cugl_conv_desc *desc)
     {
@@ -1739,6 +1794,9 @@ extern "C"
         plan->d_temp              = static_cast<uint8_t *>(d_ws);
         plan->temp_bound_bytes    = d_ws != nullptr ? bytes : 0;
         plan->core.d_rowsum_bound = plan->core.b_off != 0 ? static_cast<int32_t *>(d_ws) : nullptr;
+        plan->core.d_tmp_a_bound  = (d_ws != nullptr && plan->core.tmp_a_bytes() != 0)
+                                        ? static_cast<uint8_t *>(d_ws) + plan->core.rowsum_bytes() + plan->fold_bytes()
+                                        : nullptr;
         return CUGL_SUCCESS;
     }
 }

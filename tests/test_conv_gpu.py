@@ -95,6 +95,33 @@ def test_conv_vs_oracle(ctx, port, geom, act):
         assert np.array_equal(got, want), implicit
 
 
+@pytest.mark.parametrize("H,C,OFM,k,stride,pad,dil", [(7, 1, 5, 3, 1, 1, 1), (9, 17, 40, 3, 2, 1, 1), (8, 15, 70, 5, 1, 2, 1), (11, 33, 130, 3, 1, 0, 2),
+                                                      (6, 64, 64, 3, 1, 1, 1), (14, 100, 33, 1, 2, 0, 1), (10, 21, 30, 1, 1, 0, 1),
+                                                      (5, 130, 300, 2, 1, 1, 1), (16, 48, 48, 3, 3, 2, 1), (9, 687, 24, 5, 1, 2, 1)])
+@pytest.mark.parametrize("w_zp,in_zp", [(0, 128), (0, 0), (120, 128), (7, 0), (-9, -5)])
+def test_conv_any_channels_symmetric_and_not(ctx, port, H, C, OFM, k, stride, pad, dil, w_zp, in_zp):
+    """Channel counts that are padded to 16 (one, one over and one under a multiple) and weights with and without a zero
+    point: pixel and window sums at every border, strides that skip input pixels, dilation, patches longer than the tap
+    table of the implicit kernel (687 x 25 > 16384); implicit and explicit lowering against the oracle."""
+    signed = in_zp < 0
+    rng = np.random.default_rng(H * C + OFM)
+    t = np.int8 if signed else np.uint8
+    src = q8_uniform(rng, (3, H, H + 1, C), t)
+    wgt = q8_uniform(rng, (OFM, k, k, C), np.int8, -127, 127) if w_zp == 0 or signed else q8_uniform(rng, (OFM, k, k, C), np.uint8)
+    bias = rng.integers(-500, 501, OFM).astype(np.int32)
+    scales = np.exp(rng.uniform(np.log(1e-3), np.log(1e-2), OFM if w_zp == 0 else 1)).astype(np.float32)
+    mult, shift = f32_mults(port, 0.03, scales, 0.03 * np.sqrt(k * k * C))
+    lo, hi = type_range(t)
+    args = ((stride, stride), (pad, pad, pad, pad), in_zp, w_zp, mult, shift, 5, lo, hi)
+    want = port.conv2d_nhwc(src, wgt, bias, *args, (dil, dil))
+    pointwise = k == 1 and stride == 1
+    kernel = "gemm" if pointwise else ("implicit" if k * k * (-(-C // 16) * 16) <= 16384 else "im2col")
+    for implicit in (True, False):
+        got = gpu_conv(ctx, src, wgt, bias, *args, dilation=(dil, dil), implicit=implicit,
+                       want_kernel=kernel if implicit or pointwise else "im2col")
+        assert np.array_equal(got, want), implicit
+
+
 def test_conv_asymmetric_weights_and_signed(ctx, port):
     rng = np.random.default_rng(77)
     src = q8_uniform(rng, (2, 15, 17, 32), np.int8)
