@@ -56,6 +56,27 @@ int pick_block_n(const cugl_context *ctx, const GemmOperands &op)
     return best;
 }
 
+// CTAs that share the K range of one 64-column tile.  An output of few tiles leaves SMs idle while each busy one walks all
+// of K (about 0.2 us per 128 bytes of K); a cluster of CTAs per tile divides the walk at the price of a cluster launch and
+// one exchange of partial sums (1.5 - 2 us).  Measured, back-to-back launches, one CTA / four / eight per tile:
+// 49 x 512 x 2048: 8.0 / 7.4 / 6.8 us, 16 x 1024 x 4096: 11.6 / 8.8 / 14.4 (eight: more CTAs than SMs), 256 x 1024 x 4096
+// to float32 11.8 / 9.0, 64 x 1024 x 1024: 6.0 / 6.7; 3x3 convolutions, whose patch loads take longer, 1 x 7 x 7 x 512:
+// 18.1 / 10.7 / 8.5, 1 x 14 x 14 x 256: 11.1 / 8.8 / 7.8, 1 x 28 x 28 x 128 (K = 1152): 8.1 / 7.7 / 7.7.  Two per tile gain
+// nothing (16 x 4096 x 4096: 11.7 / 11.9).  Eight-CTA clusters need their SMs inside one GPC, hence the margins.
+int pick_split(const cugl_context *ctx, const GemmOperands &op)
+{
+    if (op.batch > 1 || op.n_extra_dst > 0 || op.channel_major > 0 || op.block_n > 0 || op.epi_warps != 0 ||
+        (op.conv != nullptr && op.conv->C == 64))
+    {
+        return 1;
+    }
+    const long long tiles = static_cast<long long>((op.M + 127) / 128) * ((op.N + 63) / 64);
+    const int       kb    = (op.K + 127) / 128;
+    if (kb >= 16 && tiles * 8 <= ctx->sm_count * 3 / 4) return 8;
+    if (kb >= (op.conv != nullptr ? 9 : 16) && tiles * 4 <= ctx->sm_count * 9 / 10) return 4;
+    return 1;
+}
+
 // the SM-pair kernel works on 256 x 256 tiles, one per pair of SMs
 bool pair_fills_the_device(const cugl_context *ctx, const GemmOperands &op)
 {
@@ -90,6 +111,13 @@ cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, c
     // stores, measured: 802816 x 256 x 64: 189 us against 170 us; 200704 x 512 x 128: 102 / 94; 50176 x 1024 x 256:
     // 57 / 60; 12544 x 2048 x 512: 37 / 43.  It needs whole 128-channel blocks (N = 64: 110 / 78).
     GemmOperands o   = op;
+    const int split = pick_split(ctx, op);
+    if (split > 1)
+    {
+        o.split_k       = split;
+        o.channel_major = -1;
+        return launch_gemmlowp_tcgen05_epi8(ctx, o, ep, false);
+    }
     o.block_n        = pick_block_n(ctx, op); // before the automatic channel-major choice below
     if (op.batch > 1)
     {

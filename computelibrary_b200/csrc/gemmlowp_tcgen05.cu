@@ -412,6 +412,8 @@ struct TileParams
     int      batch;
     int64_t  batch_dst;
     int      batch_colsum, batch_rowsum;
+    int      split;                   // kSplit instantiations: CTAs of the cluster that share one tile's K (4 or 8)
+    int      a_rows;                  // rows of an A box: 128, or fewer when M itself is smaller
     int      tma_store;               // one-CTA row-major kernels: staged groups leave as bulk tensor stores (tmap_out)
     long long spin_limit;             // clock64 ticks a wait on a barrier may last before the kernel gives up
     int      withhold_kb;             // >= 0: CTA 0 leaves out the copies of this k-block ordinal (test instrument
@@ -452,6 +454,56 @@ __device__ __forceinline__ void cluster_sync()
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr)
 {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// mbar_wait on a barrier that other CTAs of the cluster arrive on after writing to this CTA's shared memory
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t"
+                 ".reg .pred p;\n\t"
+                 "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t"
+                 "}"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int *abort_flag, int code, long long limit)
+{
+    const long long t0 = clock64();
+    while (!mbar_try_wait_cluster(bar, parity))
+    {
+        if (*abort_flag != 0)
+        {
+            return false;
+        }
+        if (clock64() - t0 > limit)
+        {
+            *abort_flag = code;
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t (&v)[32])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+                 "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]),
+                 "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]),
+                 "r"(v[30]), "r"(v[31])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait()
+{
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 // TMA tile load of a cta_group::2 pipeline: data lands in this CTA's shared memory, the byte count is
 // credited to the barrier at `bar_cluster_addr`, which lives in the leader CTA.  Not a multicast.
@@ -1663,6 +1715,79 @@ __device__ __forceinline__ void epilogue_warp_tile(uint32_t tmem_acc, const int4
     }
 }
 
+// Split-K epilogue.  The `split` CTAs of a cluster hold partial sums of one 128 x BLOCK_N tile (each over its own range of
+// K), eight warps per CTA: warp (quad, half) reads rows quad * 32 .. + 32 of column half `half`.  Every (quad, half) region
+// has one owner among the CTAs -- by column half, then by quad -- so that all of them finish a share of the tile.  A warp
+// whose region belongs to another CTA sends its 32 x BLOCK_N/2 partial sums straight into that CTA's shared memory
+// ([4 columns][lane] pieces, 512 contiguous bytes per warp store) and arrives on its barrier; the owner adds what it
+// receives to its accumulators in tensor memory (integers: exact in any order) and runs the ordinary drain on them.
+// Rows beyond M are neither sent nor drained.
+template <int BLOCK_N, bool kS32Out>
+__device__ __forceinline__ bool epilogue_warp_tile_split(uint32_t tmem_acc, const int4 *s_col, const TileParams &tp,
+                                                         const EpilogueParams &ep, int warp, int lane, int m0, int n0,
+                                                         uint8_t *out_stage, const CUtensorMap *omap, int rank, uint32_t rx,
+                                                         const uint8_t *rx_ptr, uint32_t rx_bar, volatile int *abort_flag)
+{
+    constexpr int  NH    = BLOCK_N / 2;
+    const int      quad  = warp & 3, half = (warp - kFirstEpi) >> 2;
+    const int      split = tp.split, quads_owned = 8 / split;
+    const int      owner   = half | ((split == 4 ? quad >> 1 : quad) << 1);
+    const int      q_local = split == 4 ? quad & 1 : 0;
+    const bool     live    = m0 + quad * 32 < tp.M; // warp-uniform
+    const uint32_t t_addr  = tmem_acc + (static_cast<uint32_t>(quad * 32) << 16) + half * NH;
+    uint32_t       v[32];
+    if (owner != rank)
+    {
+        if (live)
+        {
+            const int      slot = rank < owner ? rank : rank - 1;
+            const uint32_t dst  = map_to_cta(rx + static_cast<uint32_t>((slot * quads_owned + q_local) * NH * 128 + lane * 16), owner);
+#pragma unroll
+            for (int ch = 0; ch < NH / 32; ++ch)
+            {
+                tmem_ld_x32(t_addr + ch * 32, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                {
+                    st_cluster_v4(dst + (ch * 8 + j) * 512, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(rx_bar, owner));
+        return true;
+    }
+    if (!__all_sync(0xffffffffu, mbar_wait_cluster(rx_bar, 0, abort_flag, DEV_TIMEOUT_EPILOGUE, tp.spin_limit)))
+    {
+        return false;
+    }
+    if (!live)
+    {
+        return true;
+    }
+#pragma unroll
+    for (int ch = 0; ch < NH / 32; ++ch)
+    {
+        tmem_ld_x32(t_addr + ch * 32, v);
+        tmem_ld_wait();
+        for (int slot = 0; slot < split - 1; ++slot)
+        {
+            const uint4 *p = reinterpret_cast<const uint4 *>(rx_ptr + ((slot * quads_owned + q_local) * NH + ch * 32) * 128) + lane;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                const uint4 w = p[j * 32];
+                v[4 * j] += w.x, v[4 * j + 1] += w.y, v[4 * j + 2] += w.z, v[4 * j + 3] += w.w;
+            }
+        }
+        tmem_st_x32(t_addr + ch * 32, v);
+    }
+    tmem_st_wait();
+    epilogue_warp_tile<BLOCK_N, kS32Out, 1>(tmem_acc, s_col, tp, ep, warp, lane, m0, n0, out_stage, AccRelease{0u, 0u, false}, omap);
+    return true;
+}
+
 // KSUB = 128-byte K sub-blocks per pipeline stage.  One barrier hand-over (wait, MMAs, commit) costs the
 // issuing thread about 550 clocks whatever it covers, more than the 512 clocks four MMAs keep the tensor
 // cores busy, so a stage carries two sub-blocks (eight MMAs) wherever shared memory leaves room for three
@@ -1702,7 +1827,9 @@ struct SmemPlan
 // kBatched: tp.batch equal products in one launch.  A tile index then runs over (product, column block, row block),
 // row blocks fastest, so the column terms still carry over from tile to tile; operands and bulk stores go through
 // three-dimensional tensor maps, whose bounds keep a ragged last row block inside its own product.
-template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kCM, int ACC, bool kPairTma = false, bool kBatched = false>
+// kSplit: the tp.split CTAs of a cluster work on one tile, each on its own range of K (epilogue_warp_tile_split); one
+// tile per cluster.
+template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kCM, int ACC, bool kPairTma = false, bool kBatched = false, bool kSplit = false>
 __global__ void __launch_bounds__(kThreads, 1)
     gemmlowp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                             const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_res,
@@ -1733,7 +1860,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int num_n_blocks = (tp.N + BLOCK_N - 1) / BLOCK_N;
     const int num_tiles    = num_m_blocks * num_n_blocks * (kBatched ? tp.batch : 1);
     static_assert(!(kBatched && (kCM || kPairTma)), "batched launches use the row-major single-tile drain");
-    const int num_kb       = (tp.K + KSUB * BLOCK_K - 1) / (KSUB * BLOCK_K); // pipeline stages per tile
+    const int all_kb       = (tp.K + KSUB * BLOCK_K - 1) / (KSUB * BLOCK_K); // pipeline stages per tile
+    static_assert(!kSplit || (!kCM && !kPairTma && !kBatched && kEpiWarps == 8), "split K: the row-major single-tile drain of eight warps");
+    const int rank         = kSplit ? static_cast<int>(cluster_ctarank()) : 0;
+    const int kb_first     = kSplit ? rank * all_kb / tp.split : 0; // this CTA's share of them
+    const int num_kb       = kSplit ? (rank + 1) * all_kb / tp.split - kb_first : all_kb;
+    const int first_tile   = kSplit ? static_cast<int>(blockIdx.x) / tp.split : static_cast<int>(blockIdx.x);
+    const int tile_step    = kSplit ? num_tiles : static_cast<int>(gridDim.x);
+    const uint32_t rx_bar  = smem_u32(smem + P::OFF_RESBAR); // kSplit: partial sums of the other CTAs have arrived
 
     if (threadIdx.x == 0)
     {
@@ -1746,6 +1880,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         {
             mbar_init(tfull_bar(a), 1);
             mbar_init(tempty_bar(a), kEpiWarps / (kCM ? 1 : P::EPI_GROUPS)); // the warps of the group that drains it
+        }
+        if (kSplit)
+        {
+            mbar_init(rx_bar, (tp.split - 1) * (8 / tp.split)); // one arrival per source CTA and owned region
         }
         if (kPairTma)
         {
@@ -1765,6 +1903,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *s_tmem;
+    if (kSplit)
+    {
+        cluster_sync(); // barriers of every CTA are initialised before anyone arrives on them
+    }
     griddep_launch_dependents();
     griddep_wait(); // the prologue above touched no global memory
 
@@ -1778,10 +1920,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0)
         {
             const int issuer   = warp; // this warp's share of the k-block sequence
-            const int my_tiles = static_cast<int>(blockIdx.x) < num_tiles
-                                     ? (num_tiles - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1
-                                     : 0;
+            const int my_tiles = first_tile < num_tiles ? (num_tiles - 1 - first_tile) / tile_step + 1 : 0;
             const int total_kb = my_tiles * num_kb;
+            // an output of fewer than 128 rows: A boxes of that many rows (what the MMA reads of a slot's other rows only
+            // reaches accumulator rows that are never stored)
+            const uint32_t stage_bytes = kCM ? P::STAGE : KSUB * (static_cast<uint32_t>(tp.a_rows) * BLOCK_K + P::B_SUB);
             uint32_t  issued = 0, parities = 0;
             bool      ok = true;
             int       ti = 0, kb = issuer; // (tile ordinal, k-block) of g, kept incrementally
@@ -1799,7 +1942,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 {
                     break;
                 }
-                const int tile = static_cast<int>(blockIdx.x) + ti * static_cast<int>(gridDim.x);
+                const int tile = first_tile + ti * tile_step;
+                const int kg   = kb + kb_first; // k-block of the whole tile
                 const int m0   = (kCM ? tile / num_n_blocks : tile % num_m_blocks) * BLOCK_M;
                 const int nb   = kCM ? tile % num_n_blocks : tile / num_m_blocks;
                 const int z    = kBatched ? nb / num_n_blocks : 0;
@@ -1807,7 +1951,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (kb == 0) trace_event(tp.trace, ti, 0);
                 if (kBatched)
                 {
-                    mbar_expect_tx(full_bar(st), P::STAGE);
+                    mbar_expect_tx(full_bar(st), stage_bytes);
 #pragma unroll
                     for (int sub = 0; sub < KSUB; ++sub)
                     {
@@ -1827,13 +1971,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const int n  = fast_div(t, tp.conv_div_ho);
                     const int pp = t - n * tp.conv_ho;
                     const int w0 = q * tp.conv_sx - tp.conv_pl, h0 = pp * tp.conv_sy - tp.conv_pt;
-                    const int left  = (tp.K - kb * KSUB * BLOCK_K + BLOCK_K - 1) / BLOCK_K;
+                    const int left  = (tp.K - kg * KSUB * BLOCK_K + BLOCK_K - 1) / BLOCK_K;
                     const int valid = left < KSUB ? left : KSUB;
                     if (tp.conv_c == 64)
                     {
                         // 64 channels: a 128-byte K block is two filter taps, loaded as two tiles of 128 pixels x 64 bytes
                         // (64-byte swizzle) one behind the other; the last block of an odd tap count holds one
-                        const int taps_left = (tp.K >> 6) - 2 * kb * KSUB;
+                        const int taps_left = (tp.K >> 6) - 2 * kg * KSUB;
                         const int taps      = taps_left < 2 * KSUB ? taps_left : 2 * KSUB;
                         mbar_expect_tx(full_bar(st), taps * (A_STAGE / 2) + valid * P::B_SUB);
 #pragma unroll
@@ -1841,7 +1985,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         {
                             if (j < taps)
                             {
-                                const int tap = 2 * kb * KSUB + j;
+                                const int tap = 2 * kg * KSUB + j;
                                 const int ky = tap / tp.conv_kw, kx = tap - ky * tp.conv_kw;
                                 tma_load_im2col(sA + st * P::A_STAGE_K + j * (A_STAGE / 2), &tmap_a, 0, w0, h0, n,
                                                 static_cast<uint16_t>(kx * tp.conv_dx),
@@ -1853,7 +1997,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         {
                             if (sub < valid)
                             {
-                                tma_load_2d(sB + st * P::B_STAGE + sub * P::B_SUB, &tmap_b, (kb * KSUB + sub) * BLOCK_K, n0,
+                                tma_load_2d(sB + st * P::B_STAGE + sub * P::B_SUB, &tmap_b, (kg * KSUB + sub) * BLOCK_K, n0,
                                             full_bar(st));
                             }
                         }
@@ -1866,7 +2010,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         {
                             if (sub < valid)
                             {
-                                const int k0  = (kb * KSUB + sub) * BLOCK_K;
+                                const int k0  = (kg * KSUB + sub) * BLOCK_K;
                                 const int tap = k0 / tp.conv_c, c0 = k0 - tap * tp.conv_c;
                                 const int ky = tap / tp.conv_kw, kx = tap - ky * tp.conv_kw;
                                 tma_load_im2col(sA + st * P::A_STAGE_K + sub * A_STAGE, &tmap_a, c0, w0, h0, n,
@@ -1881,11 +2025,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 else if (g != tp.withhold_kb || blockIdx.x != 0)
                 {
-                    mbar_expect_tx(full_bar(st), P::STAGE);
+                    mbar_expect_tx(full_bar(st), stage_bytes);
 #pragma unroll
                     for (int sub = 0; sub < KSUB; ++sub)
                     {
-                        const int k0 = (kb * KSUB + sub) * BLOCK_K; // beyond K: the copy delivers zeros
+                        const int k0 = (kg * KSUB + sub) * BLOCK_K; // beyond K: the copy delivers zeros
                         tma_load_2d(sA + st * P::A_STAGE_K + sub * A_STAGE, &tmap_a, k0, m0, full_bar(st));
                         tma_load_2d(sB + st * P::B_STAGE + sub * P::B_SUB, &tmap_b, k0, n0, full_bar(st));
                     }
@@ -1943,7 +2087,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool     a_sw64  = !kCM && tp.conv_c == 64;
             const uint64_t a_desc0 = a_sw64 ? make_kmajor_sw64_desc(sA) : make_kmajor_sw128_desc(sA);
             const uint64_t b_desc0 = make_kmajor_sw128_desc(sB);
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti)
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++ti)
             {
                 ok = mbar_wait(tempty_bar(as), aph ^ 1, s_abort, DEV_TIMEOUT_MMA, tp.spin_limit);
                 if (!ok)
@@ -1984,7 +2128,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     // A stage wholly inside K and 128-byte-swizzle operands (the common case): the MMAs back to back with
                     // nothing to test on the issuing thread's critical path.  Else the K steps beyond K are left out (zero
                     // fill, or with im2col-mode loads not loaded at all) and 64-byte-swizzle A tiles are addressed tap by tap.
-                    if ((kb + 1) * KSUB * BLOCK_K <= tp.K && !a_sw64)
+                    if ((kb_first + kb + 1) * KSUB * BLOCK_K <= tp.K && !a_sw64)
                     {
 #pragma unroll
                         for (int sub = 0; sub < KSUB; ++sub)
@@ -2006,7 +2150,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                             for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
                             {
-                                if ((kb * KSUB + sub) * BLOCK_K + k * UMMA_K < tp.K)
+                                if (((kb_first + kb) * KSUB + sub) * BLOCK_K + k * UMMA_K < tp.K)
                                 {
                                     // 32 bytes on inside the swizzled row: + 2; 64-byte rows: the next tap's tile after two steps
                                     const uint32_t a_k = a_sw64 ? static_cast<uint32_t>((k >> 1) * ((A_STAGE / 2) >> 4) + 2 * (k & 1))
@@ -2042,7 +2186,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---------------------------------------------------------------- epilogue (warps 2..9)
         // One group of all epilogue warps, or (narrow tiles, eight warps) two groups of four draining alternate
         // tiles: accumulator buffer and phase follow from the tile ordinal, so the groups need not talk.
-        constexpr int kGroups = kCM ? 1 : P::EPI_GROUPS;
+        constexpr int kGroups = kCM || kSplit ? 1 : P::EPI_GROUPS;
         const int     group   = kGroups == 1 ? 0 : (warp - kFirstEpi) >> 2;
         const int     et      = threadIdx.x - 32 * kFirstEpi - group * 128; // thread index inside the group
         int4         *g_col   = s_col + group * BLOCK_N;
@@ -2058,10 +2202,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         constexpr int  kStride  = 1;
         // Two buffers only: with 128-column tiles in four buffers, pairs (0, 1) and (2, 3) drained by sixteen warps while
         // the MMA warp fills the other pair, the same layers measured slower (802816 x 256 x 64: 164 against 133 us).
-        constexpr bool kCanPair = !kCM && !kS32Out && kGroups == 1 && ACC == 2 && !kBatched;
+        constexpr bool kCanPair = !kCM && !kS32Out && kGroups == 1 && ACC == 2 && !kBatched && !kSplit;
         int            skip     = -1; // ordinal of a tile already drained as the partner of an earlier one
         uint32_t       n_res_pairs = 0; // kPairTma: pairs whose residual this warp has fetched (phase of its barrier)
-        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++ti)
+        for (int tile = first_tile; tile < num_tiles; tile += tile_step, ++ti)
         {
             if ((kGroups > 1 && (ti & 1) != group) || ti == skip)
             {
@@ -2151,6 +2295,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                                                             smem + P::OFF_OUT);
                     release_accumulators(rel, lane);
                 }
+                else if constexpr (kSplit)
+                {
+                    ok = epilogue_warp_tile_split<BLOCK_N, kS32Out>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane, m0, n0,
+                                                                    smem + P::OFF_OUT, tp.tma_store != 0 ? &tmap_out : nullptr, rank,
+                                                                    smem_u32(smem + P::TOTAL), smem + P::TOTAL, rx_bar, s_abort);
+                }
                 else if (kCanPair && pair_now)
                 {
                     epilogue_warp_tile_pair<BLOCK_N, kGroups>(tmem_base + as * BLOCK_N, tmem_base + (as + kStride) * BLOCK_N,
@@ -2201,6 +2351,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---------------------------------------------------------------- teardown
     tc_fence_before();
     __syncthreads();
+    if (kSplit)
+    {
+        cluster_sync(); // nobody leaves while a peer may still write into its shared memory (every wait above is bounded)
+    }
     if (warp == kMmaWarp)
     {
         tc_fence_after();
@@ -3236,15 +3390,18 @@ bool conv_tma_supported(const GemmOperands &op)
            (cv.kw - 1) * cv.dil_x < 256 && (cv.kh - 1) * cv.dil_y < 256 && get_encode_im2col_fn() != nullptr;
 }
 
-template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kPairTma = false, bool kBatched = false>
+template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kPairTma = false, bool kBatched = false, bool kSplit = false>
 cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
 {
     constexpr int ACC = BLOCK_N <= 128 ? 4 : 2; // narrow tiles: four accumulator buffers in the 512 columns
     using P = SmemPlan<BLOCK_N, STAGES, KSUB, ACC, kPairTma>;
-    static_assert(P::DYN_BYTES <= 227 * 1024, "shared memory plan exceeds the sm_100 limit");
+    // kSplit: room for the partial sums a CTA receives, split - 1 times a 1/split share of the tile
+    constexpr int kDynBytes = P::DYN_BYTES + (kSplit ? BLOCK_M * BLOCK_N * 4 * 7 / 8 : 0);
+    static_assert(kDynBytes <= 227 * 1024, "shared memory plan exceeds the sm_100 limit");
+    const int a_rows = op.conv == nullptr && op.M < BLOCK_M ? (op.M + 7) / 8 * 8 : BLOCK_M; // whole 8-row swizzle groups
     CUtensorMap map_a, map_b;
     if (!(op.conv != nullptr ? encode_im2col_map(&map_a, *op.conv)
-                             : encode_operand_map(&map_a, op.a, op.M, op.K, op.lda, BLOCK_M, kBatched ? op.batch : 0, op.a_batch_stride)) ||
+                             : encode_operand_map(&map_a, op.a, op.M, op.K, op.lda, a_rows, kBatched ? op.batch : 0, op.a_batch_stride)) ||
         !encode_operand_map(&map_b, op.bt, op.N, op.K, op.ldbt, BLOCK_N, kBatched ? (op.bt_batch_stride != 0 ? op.batch : 1) : 0,
                             op.bt_batch_stride != 0 ? op.bt_batch_stride : op.ldbt * op.N))
     {
@@ -3267,11 +3424,11 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
             return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the residual tiles");
         }
     }
-    auto kernel = gemmlowp_tcgen05_kernel<BLOCK_N, STAGES, KSUB, kS32Out, false, ACC, kPairTma, kBatched>;
+    auto kernel = gemmlowp_tcgen05_kernel<BLOCK_N, STAGES, KSUB, kS32Out, false, ACC, kPairTma, kBatched, kSplit>;
     static bool attr_set[64] = {}; // per instantiation and device
     if (!attr_set[ctx->device & 63])
     {
-        CUGL_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::DYN_BYTES));
+        CUGL_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynBytes));
         attr_set[ctx->device & 63] = true;
     }
     TileParams tp;
@@ -3302,7 +3459,9 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
     {
         return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "more than 2^31 output tiles");
     }
-    const int grid  = units < ctx->sm_count ? static_cast<int>(units) : ctx->sm_count;
+    tp.split  = kSplit ? op.split_k : 1;
+    tp.a_rows = a_rows;
+    const int grid  = kSplit ? tiles * op.split_k : units < ctx->sm_count ? static_cast<int>(units) : ctx->sm_count;
     tp.tma_store = tma_store ? 1 : 0;
     tp.batch     = kBatched ? op.batch : 1;
     tp.batch_dst = op.d_batch_stride;
@@ -3312,7 +3471,7 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
     {
         tp.pair_drain = 0;
     }
-    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, kernel, grid, kThreads, P::DYN_BYTES, map_a, map_b, map_out, map_res, tp, ep));
+    CUGL_CUDA_TRY(ctx, launch_dependent_cluster(ctx, kernel, grid, kThreads, kDynBytes, kSplit ? op.split_k : 1, map_a, map_b, map_out, map_res, tp, ep));
     return check_cuda(ctx, cudaGetLastError(), "gemmlowp_tcgen05_kernel");
 }
 
@@ -3553,6 +3712,14 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
             return s32 ? launch_variant<64, 4, 2, true, false, true>(ctx, op, ep) : launch_variant<64, 4, 2, false, false, true>(ctx, op, ep);
         }
         return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "batched launches belong to the eight-warp build");
+    }
+    if (op.split_k > 1)
+    {
+        if constexpr (kEpiWarps == 8)
+        {
+            return s32 ? launch_variant<64, 6, 1, true, false, false, true>(ctx, op, ep) : launch_variant<64, 6, 1, false, false, false, true>(ctx, op, ep);
+        }
+        return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "split-K launches belong to the eight-warp build");
     }
     // channel-major accumulators: no row-sum term (it would be a per-column quantity there) and one destination
     if (op.channel_major > 0 && ep.rowsum == nullptr && op.n_extra_dst == 0 && op.conv == nullptr)

@@ -101,6 +101,9 @@ struct GemmOperands
     // the same kernels: < 0 keeps 128-row units of work; otherwise 256-row units (two tiles per hand-over) where the
     // output is large enough
     int double_tile;
+    // one-CTA row-major kernels with 64-column tiles: 4 or 8 CTAs (a cluster) share the K range of every tile; 0 / 1: no.
+    // Set by the dispatcher.
+    int split_k;
     // one-CTA row-major kernels: > 1 runs that many products of M x N x K in one launch.  Byte distances between
     // consecutive products; bt_batch_stride = 0 shares one Bt.  The row sums of product i start at entry i * M of the
     // row-sum vector, its column sums at entry i * N (0 when Bt is shared).  No residual, no extra destinations.
@@ -184,18 +187,37 @@ inline bool use_dependent_launch(const cugl_context *ctx)
 // Launch with programmatic stream serialization (griddepcontrol in the kernel): the kernel may start its prologue while the
 // previous kernel of the stream is finishing.  ctx->dependent_launch == 0 or a capturing stream: a plain launch.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(cugl_context *ctx, void (*kernel)(KArgs...), int grid, int threads, int smem_bytes, Args &&...args)
+cudaError_t launch_dependent_cluster(cugl_context *ctx, void (*kernel)(KArgs...), int grid, int threads, int smem_bytes, int cluster,
+                                     Args &&...args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim          = dim3(static_cast<unsigned>(grid), 1, 1);
     cfg.blockDim         = dim3(static_cast<unsigned>(threads), 1, 1);
     cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
     cfg.stream           = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int                 n = 0;
+    if (cluster > 1)
+    {
+        attr[n].id               = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = static_cast<unsigned>(cluster);
+        attr[n].val.clusterDim.y = 1;
+        attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (use_dependent_launch(ctx))
+    {
+        attr[n].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
     cfg.attrs    = attr;
-    cfg.numAttrs = use_dependent_launch(ctx) ? 1 : 0;
+    cfg.numAttrs = static_cast<unsigned>(n);
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(cugl_context *ctx, void (*kernel)(KArgs...), int grid, int threads, int smem_bytes, Args &&...args)
+{
+    return launch_dependent_cluster(ctx, kernel, grid, threads, smem_bytes, 1, static_cast<Args &&>(args)...);
 }
 } // namespace cugl

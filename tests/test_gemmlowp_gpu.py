@@ -174,6 +174,53 @@ def test_operand_preparation(ctx, port, M, N, K):
             assert np.array_equal(acc, port.gemmlowp_core(a, b, 11, -7))
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 64, 2048), (33, 65, 2100), (49, 512, 4608), (97, 31, 16000), (130, 500, 1300), (300, 600, 2000),
+                                   (256, 900, 2176), (128, 2112, 2048), (128, 2113, 2048), (128, 8, 2047)])
+def test_split_k(ctx, port, M, N, K):
+    """Outputs of few tiles, whose K range is shared by clusters of 4 and 8 CTAs: ragged rows, columns and K, K ranges
+    that do not divide evenly, every output type and stage encoding, against the oracle and the one-CTA kernel."""
+    rng = np.random.default_rng(M + N + K)
+    for t, a_off, b_off in ((np.uint8, -128, -120), (np.int8, 5, 0)):
+        a, b = q8_uniform(rng, (M, K), t), q8_uniform(rng, (K, N), t)
+        lo, hi = type_range(t)
+        bias = rng.integers(-2000, 2001, N).astype(np.int32)
+        ms = [capi.calculate_quantized_multiplier(np.float32(x / (73 * np.sqrt(K)))) for x in rng.uniform(0.2, 1.0, N)]
+        mult, shift = np.array([m for m, _ in ms], np.int32), np.array([s for _, s in ms], np.int32)
+        if b_off != 0:
+            mult, shift = mult[:1], shift[:1]
+        args = (a, b, bias, a_off, b_off, mult if b_off == 0 else int(mult[0]), shift if b_off == 0 else int(shift[0]), 3, lo, hi, t)
+        want = port.gemmlowp_fused(a, b, bias, a_off, b_off, mult, shift, 3, lo, hi, t)
+        for pad in (0, 5):
+            got, _ = gpu_gemmlowp(ctx, *args, ldd_pad=pad, runs=2)
+            assert np.array_equal(got, want), (t, pad)
+        one, _ = gpu_gemmlowp(ctx, *args, tile_columns=64)
+        assert np.array_equal(one, want)
+        core = port.gemmlowp_core(a, b, a_off, b_off)
+        acc, _ = gpu_gemmlowp(ctx, a, b, None, a_off, b_off, 0, 0, 0, 0, 0, np.int32, ldd_pad=4)
+        assert np.array_equal(acc, core)
+        init = rng.integers(-1000, 1001, (M, N)).astype(np.int32)
+        acc, _ = gpu_gemmlowp(ctx, a, b, None, a_off, b_off, 0, 0, 0, 0, 0, np.int32, accumulate=True, dst_init=init)
+        assert np.array_equal(acc, core + init)
+        f, _ = gpu_gemmlowp(ctx, a, b, None, a_off, b_off, 0, 0, 0, 0, 0, np.float32, dequantize_scale=0.37e-3)
+        assert np.array_equal(f, core.astype(np.float32) * np.float32(0.37e-3))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4, 16), (130, 36, 100), (257, 260, 300), (129, 132, 1500), (1000, 516, 1056), (700, 2052, 144),
+                                   (2500, 2052, 1040), (64, 33, 64)])
+@pytest.mark.parametrize("ldd_pad", [0, 4])
+def test_32_bit_results_through_bulk_stores(ctx, port, M, N, K, ldd_pad):
+    """S32 and F32 destinations leave as bulk tensor stores where N and the pitch allow it: every tile width and kernel,
+    ragged edges with canary bytes behind each row, against the oracle and the per-lane stores."""
+    rng = np.random.default_rng(M + N + K)
+    a, b = q8_uniform(rng, (M, K), np.int8), q8_uniform(rng, (K, N), np.int8)
+    core = port.gemmlowp_core(a, b, 7, -3)
+    for store in (True, False):
+        acc, _ = gpu_gemmlowp(ctx, a, b, None, 7, -3, 0, 0, 0, 0, 0, np.int32, ldd_pad=ldd_pad, tma_store=store)
+        assert np.array_equal(acc, core), store
+        f, _ = gpu_gemmlowp(ctx, a, b, None, 7, -3, 0, 0, 0, 0, 0, np.float32, ldd_pad=ldd_pad, dequantize_scale=1.3e-4, tma_store=store)
+        assert np.array_equal(f, core.astype(np.float32) * np.float32(1.3e-4)), store
+
+
 def test_run_twice_and_variable_b(ctx, port):
     """MultipleExecution (GEMMLowp.cpp:211-297): same plan, same output; B re-laid out per run when it is
     not constant (reshape_b_only_on_first_run = false)."""
