@@ -151,7 +151,7 @@ cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, c
     // sixteen epilogue warps (256-column tiles only) buy another 4 - 7 % on short K with wide outputs
     // (up to K = 512, where its paired drain applies; above, eight warps -- whose single-tile drain stores through the
     // TMA unit -- measured faster: 50176 x 256 x 1024 25.5 against 27.6 us)
-    if (o.N > 128 && (o.epi_warps == 16 || (o.epi_warps != 4 && o.epi_warps != 8 && o.K <= 512)))
+    if (o.N > 128 && (o.epi_warps == 16 || (ep.stage != CUGL_STAGE_NONE && o.epi_warps != 4 && o.epi_warps != 8 && o.K <= 512)))
     {
         return launch_gemmlowp_tcgen05_epi16(ctx, o, ep, false);
     }

@@ -747,6 +747,7 @@ constexpr int kOutPieces     = kOutRowBytes / 16;
 constexpr int kOutChunks     = kOutRowBytes / 32; // 32-column chunks per staged group
 constexpr int kCmPitchWords  = 36;                // channel-major transpose stage (store_chunk_cm_staged)
 constexpr int kCmStageBytes  = 8 * kCmPitchWords * 4;
+constexpr int kRawStageBytes = 32 * 128;          // 32-bit results: 32 rows x 32 columns
 constexpr int kOutStageBytes = 32 * kOutRowBytes > kCmStageBytes ? 32 * kOutRowBytes : kCmStageBytes;
 
 // Swizzle of the staged rows.  The library's own flush reads the stage back with any conflict-free pattern (row & mask);
@@ -933,6 +934,35 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
     const bool    tma     = !kS32Out && omap != nullptr && tp.n_extra == 0; // warp-uniform
     const bool    staged  = !kS32Out && (tp.n_extra > 0 || tma);            // warp-uniform
     // chunk c of the warp's columns into the stage; the group goes out when it is complete
+    // 32-bit results: a chunk of 32 rows x 128 bytes leaves as one bulk tensor store as well.  A lane's own stores are
+    // 16-byte pieces of one row each, a row pitch apart: eight times the load/store passes, and half a sector each.
+    const bool    raw_tma = kS32Out && omap != nullptr; // warp-uniform (encode_raw_map: one destination, no accumulation)
+    auto raw_stage_and_flush = [&](const uint32_t *v, int c) {
+        if (n_first + c * 32 >= tp.N)
+        {
+            return;
+        }
+        stage_reuse_wait(lane);
+        const bool     to_f32 = tp.raw_f32 != 0;
+        EpilogueParams rp{};
+        rp.out_f32  = 1;
+        rp.dq_scale = tp.raw_scale;
+        uint8_t *row = stage + lane * 128;
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+        {
+            uint4 w = make_uint4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]);
+            if (to_f32)
+            {
+                w.x = raw_result_word(static_cast<int32_t>(w.x), 0u, rp);
+                w.y = raw_result_word(static_cast<int32_t>(w.y), 0u, rp);
+                w.z = raw_result_word(static_cast<int32_t>(w.z), 0u, rp);
+                w.w = raw_result_word(static_cast<int32_t>(w.w), 0u, rp);
+            }
+            *reinterpret_cast<uint4 *>(row + ((p ^ (lane & 7)) << 4)) = w; // the 128-byte swizzle of the map
+        }
+        flush_stage_tma(stage, omap, m - lane, n_first + c * 32, lane, z);
+    };
     auto stage_and_flush = [&](const uint32_t *v, int c) {
         const int gc = c & (kOutChunks - 1);
         if (tma && gc == 0)
@@ -982,7 +1012,11 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
             load_residual(res, tp.residual + row_off, n_first + ch * 32, row_ok, tp);
             add_residual(va, res, tp);
         }
-        if (staged)
+        if (raw_tma)
+        {
+            raw_stage_and_flush(va, ch);
+        }
+        else if (staged)
         {
             stage_and_flush(va, ch);
         }
@@ -1012,7 +1046,11 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
                 load_residual(res, tp.residual + row_off, n_first + (ch + 1) * 32, row_ok, tp);
                 add_residual(vb, res, tp);
             }
-            if (staged)
+            if (raw_tma)
+            {
+                raw_stage_and_flush(vb, ch + 1);
+            }
+            else if (staged)
             {
                 stage_and_flush(vb, ch + 1);
             }
@@ -1681,7 +1719,7 @@ __device__ __forceinline__ void epilogue_warp_tile(uint32_t tmem_acc, const int4
                                                    int32_t given_row_term = 0)
 {
     constexpr int NCOLS    = BLOCK_N * kGroups / (kEpiWarps / 4);
-    uint8_t      *stage    = out_stage + (warp - kFirstEpi) * kOutStageBytes;
+    uint8_t      *stage    = out_stage + (warp - kFirstEpi) * (kS32Out && kEpiWarps <= 8 ? kRawStageBytes : kOutStageBytes);
     const int     quad     = warp & 3;               // tensor-memory lane quarter this warp may read
     const int     half     = kGroups == 1 ? (warp - kFirstEpi) >> 2 : 0; // which share of the columns
     const int     m        = m0 + quad * 32 + lane;
@@ -1794,9 +1832,11 @@ __device__ __forceinline__ bool epilogue_warp_tile_split(uint32_t tmem_acc, cons
 // such stages.
 // RESB > 0 (implicit convolution with one column block): the whole B operand stays in RESB bytes of shared memory for
 // the life of the CTA and the ring holds A stages only.
-template <int BLOCK_N, int STAGES, int KSUB, int ACC = 2, bool kPairTma = false, int RESB = 0>
+// RAW: 32-bit results, staged 32 rows x 128 bytes per warp whatever the warp count.
+template <int BLOCK_N, int STAGES, int KSUB, int ACC = 2, bool kPairTma = false, int RESB = 0, bool RAW = false>
 struct SmemPlan
 {
+    static constexpr int OUT_STAGE  = RAW ? kRawStageBytes : (kPairTma ? kPairStageBytes : kOutStageBytes); // per epilogue warp
     static constexpr int ACC_STAGES = ACC; // accumulator buffers in tensor memory (ACC * BLOCK_N <= 512 columns)
     static_assert(ACC * BLOCK_N <= 512 && (ACC == 2 || ACC == 4), "tensor memory holds 512 columns");
     static_assert(STAGES >= kProdLanes, "the producer lanes of one round must own distinct stages");
@@ -1815,7 +1855,7 @@ struct SmemPlan
     static constexpr int OFF_RESBAR = OFF_MISC + 16;              // kPairTma: one barrier per epilogue warp (residual boxes)
     static constexpr int OFF_OUT    = ((OFF_RESBAR + 8 * kEpiWarps + 1023) / 1024) * 1024;
     // kPairTma: the paired drain stages two tiles of 32 rows x 64 bytes per warp for its bulk tensor stores
-    static constexpr int TOTAL      = OFF_OUT + kEpiWarps * (kPairTma ? kPairStageBytes : kOutStageBytes);
+    static constexpr int TOTAL      = OFF_OUT + kEpiWarps * OUT_STAGE;
     static constexpr int DYN_BYTES  = TOTAL + 1024;               // slack to align the base to 1024
     static constexpr int TMEM_COLS  = ACC * BLOCK_N;
 };
@@ -1835,7 +1875,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                             const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_res,
                             const __grid_constant__ TileParams tp, const EpilogueParams ep)
 {
-    using P = SmemPlan<BLOCK_N, STAGES, KSUB, ACC, kPairTma>;
+    using P = SmemPlan<BLOCK_N, STAGES, KSUB, ACC, kPairTma, 0, kS32Out && !kCM && kEpiWarps <= 8>;
     extern __shared__ uint8_t smem_raw[];
     // the 1024-byte aligned start of the dynamic shared memory, derived by pointer arithmetic on the __shared__ array
     // itself: a pointer rebuilt from an integer loses its address space and every access through it becomes a
@@ -3335,6 +3375,28 @@ bool encode_out_map(const GemmOperands &op, CUtensorMap *map, bool *use, int row
               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same for 32-bit results: boxes of 32 x 32 elements.  Not for dst += result; N a multiple of four (a bulk store clips at
+// the end of a row in whole 16-byte units).
+bool encode_raw_map(const GemmOperands &op, const EpilogueParams &ep, CUtensorMap *map, bool *use)
+{
+    const bool batched = op.batch > 1;
+    *use = kEpiWarps <= 8 && op.tma_store >= 0 && op.n_extra_dst == 0 && ep.accumulate == 0 && (op.N & 3) == 0 &&
+           ((reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd) |
+             (batched ? static_cast<uint64_t>(op.d_batch_stride) : 0)) & 15) == 0;
+    if (!*use)
+    {
+        return true;
+    }
+    EncodeTiledFn    fn         = get_encode_fn();
+    const cuuint64_t dims[3]    = {static_cast<cuuint64_t>(op.N), static_cast<cuuint64_t>(op.M), static_cast<cuuint64_t>(op.batch)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(op.ldd), static_cast<cuuint64_t>(op.d_batch_stride)};
+    const cuuint32_t box[3]     = {32, 32, 1};
+    const cuuint32_t estr[3]    = {1, 1, 1};
+    return fn != nullptr && fn(map, CU_TENSOR_MAP_DATA_TYPE_INT32, batched ? 3 : 2, op.dst, dims, strides, box, estr,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 using EncodeIm2colFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                     const cuuint64_t *, const int *, const int *, cuuint32_t, cuuint32_t,
                                     const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -3394,7 +3456,7 @@ template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kPairTma = false
 cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
 {
     constexpr int ACC = BLOCK_N <= 128 ? 4 : 2; // narrow tiles: four accumulator buffers in the 512 columns
-    using P = SmemPlan<BLOCK_N, STAGES, KSUB, ACC, kPairTma>;
+    using P = SmemPlan<BLOCK_N, STAGES, KSUB, ACC, kPairTma, 0, kS32Out && kEpiWarps <= 8>;
     // kSplit: room for the partial sums a CTA receives, split - 1 times a 1/split share of the tile
     constexpr int kDynBytes = P::DYN_BYTES + (kSplit ? BLOCK_M * BLOCK_N * 4 * 7 / 8 : 0);
     static_assert(kDynBytes <= 227 * 1024, "shared memory plan exceeds the sm_100 limit");
@@ -3410,6 +3472,10 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
     CUtensorMap map_out   = map_a; // placeholder when unused
     bool        tma_store = false;
     if (!kS32Out && !(kPairTma ? encode_out_map(op, &map_out, &tma_store, 64, true) : encode_out_map(op, &map_out, &tma_store)))
+    {
+        return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the output tiles");
+    }
+    if (kS32Out && !encode_raw_map(op, ep, &map_out, &tma_store))
     {
         return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the output tiles");
     }
@@ -3538,6 +3604,10 @@ cugl_status launch_variant_2cta(cugl_context *ctx, const GemmOperands &op, const
     CUtensorMap map_out   = map_a; // placeholder when unused
     bool        tma_store = false;
     if (!kS32Out && !encode_out_map(op, &map_out, &tma_store))
+    {
+        return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the output tiles");
+    }
+    if (kS32Out && kEpiWarps == 4 && !encode_raw_map(op, ep, &map_out, &tma_store)) // (four warps: their staging has the size)
     {
         return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the output tiles");
     }
@@ -3707,9 +3777,9 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
         if constexpr (kEpiWarps == 8)
         {
             const int bn = op.block_n > 0 ? op.block_n : (op.N > 128 ? 256 : (op.N > 64 ? 128 : 64));
-            if (bn > 128) return s32 ? launch_variant<256, 4, 1, true, false, true>(ctx, op, ep) : launch_variant<256, 4, 1, false, false, true>(ctx, op, ep);
-            if (bn > 64) return s32 ? launch_variant<128, 3, 2, true, false, true>(ctx, op, ep) : launch_variant<128, 3, 2, false, false, true>(ctx, op, ep);
-            return s32 ? launch_variant<64, 4, 2, true, false, true>(ctx, op, ep) : launch_variant<64, 4, 2, false, false, true>(ctx, op, ep);
+            if (bn > 128) return s32 ? launch_variant<256, 3, 1, true, false, true>(ctx, op, ep) : launch_variant<256, 4, 1, false, false, true>(ctx, op, ep);
+            if (bn > 64) return s32 ? launch_variant<128, 5, 1, true, false, true>(ctx, op, ep) : launch_variant<128, 3, 2, false, false, true>(ctx, op, ep);
+            return s32 ? launch_variant<64, 3, 2, true, false, true>(ctx, op, ep) : launch_variant<64, 4, 2, false, false, true>(ctx, op, ep);
         }
         return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "batched launches belong to the eight-warp build");
     }
@@ -3717,7 +3787,7 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
     {
         if constexpr (kEpiWarps == 8)
         {
-            return s32 ? launch_variant<64, 6, 1, true, false, false, true>(ctx, op, ep) : launch_variant<64, 6, 1, false, false, false, true>(ctx, op, ep);
+            return s32 ? launch_variant<64, 5, 1, true, false, false, true>(ctx, op, ep) : launch_variant<64, 6, 1, false, false, false, true>(ctx, op, ep);
         }
         return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "split-K launches belong to the eight-warp build");
     }
@@ -3746,7 +3816,8 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
 #endif
     if (block_n > 128 || !CUGL_TC_FULL_BUILD)
     {
-        return s32 ? launch_variant<256, 4, 1, true>(ctx, op, ep) : launch_variant<256, 4, 1, false>(ctx, op, ep);
+        constexpr int kRawStages = kEpiWarps == 8 ? 3 : 4; // (eight warps stage 32 KB of 32-bit results)
+        return s32 ? launch_variant<256, kRawStages, 1, true>(ctx, op, ep) : launch_variant<256, 4, 1, false>(ctx, op, ep);
     }
 #if CUGL_TC_FULL_BUILD
     // K of at most one 128-byte block: a tile is a single stage, so one-block stages and a ring twice as deep keep
@@ -3755,10 +3826,15 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
     if (block_n > 64)
     {
         if (one_block) return launch_variant<128, 6, 1, false>(ctx, op, ep);
-        return s32 ? launch_variant<128, 3, 2, true>(ctx, op, ep) : launch_variant<128, 3, 2, false>(ctx, op, ep);
+        if (s32)
+        {
+            if constexpr (kEpiWarps == 4) return launch_variant<128, 3, 2, true>(ctx, op, ep);
+            else return launch_variant<128, 5, 1, true>(ctx, op, ep);
+        }
+        return launch_variant<128, 3, 2, false>(ctx, op, ep);
     }
     if (one_block) return launch_variant<64, 8, 1, false>(ctx, op, ep);
-    return s32 ? launch_variant<64, 4, 2, true>(ctx, op, ep) : launch_variant<64, 4, 2, false>(ctx, op, ep);
+    return s32 ? launch_variant<64, 3, 2, true>(ctx, op, ep) : launch_variant<64, 4, 2, false>(ctx, op, ep);
 #endif
 }
 } // namespace cugl
