@@ -457,6 +457,9 @@ __global__ void __launch_bounds__(kThreads) output_stage_kernel(const int32_t *_
                                                                 int32_t shift, int32_t offset, int32_t lo, int32_t hi,
                                                                 bool vec_ok, bool integer_stage)
 {
+    // behind the product that writes its input: scheduled while that kernel finishes, no access before it has
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int n0 = (blockIdx.x * kThreads + threadIdx.x) * 4;
     if (n0 >= N)
     {
@@ -866,15 +869,15 @@ cugl_status launch_output_stage(cugl_context *ctx, const int32_t *d_in, int64_t 
     const dim3 blocks(gx, gy);
     if (out16)
     {
-        output_stage_kernel<true><<<blocks, kThreads, 0, ctx->stream>>>(
+        CUGL_CUDA_TRY(ctx, launch_dependent(ctx, output_stage_kernel<true>, blocks, kThreads, 0,
             d_in, ld_in_bytes / 4, d_bias, static_cast<uint8_t *>(d_out), ld_out_bytes, M, N, d_mults, d_shifts, mult,
-            shift, offset, lo, hi, vec_ok, integer_stage);
+            shift, offset, lo, hi, vec_ok, integer_stage));
     }
     else
     {
-        output_stage_kernel<false><<<blocks, kThreads, 0, ctx->stream>>>(
+        CUGL_CUDA_TRY(ctx, launch_dependent(ctx, output_stage_kernel<false>, blocks, kThreads, 0,
             d_in, ld_in_bytes / 4, d_bias, static_cast<uint8_t *>(d_out), ld_out_bytes, M, N, d_mults, d_shifts, mult,
-            shift, offset, lo, hi, vec_ok, integer_stage);
+            shift, offset, lo, hi, vec_ok, integer_stage));
     }
     return check_cuda(ctx, cudaGetLastError(), "output_stage_kernel");
 }

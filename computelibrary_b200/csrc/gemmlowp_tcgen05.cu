@@ -766,45 +766,96 @@ __device__ __forceinline__ void stage_chunk(uint8_t *stage, const uint32_t *w, i
     *reinterpret_cast<uint4 *>(row + (((2 * group_chunk + 1) ^ sw) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
-__device__ __forceinline__ void flush_stage(const uint8_t *stage, const TileParams &tp, int m_base, int n_group,
-                                            int ncols_group, int lane, bool tma = false, int64_t dst_off = 0)
+// d0: first valid byte of row 0 in global memory (16-byte aligned rows); rows, n: valid rows and bytes per row.  A call of its
+// own, everything by value, like the two below: the drain is instantiated for every encoding, and its code is fetched afresh
+// by every launch -- with the store paths inlined a ResNet-50 layer at batch 256 started about 0.6 us later.
+__device__ __noinline__ void flush_stage(const uint8_t *stage, uint8_t *d0, int64_t ldd, int rows, int n, int lane, bool tma)
 {
     __syncwarp();
     const int p = lane & (kOutPieces - 1);
 #pragma unroll 2
-    for (int it = 0; it < kOutPieces; ++it)
+    for (int r = lane / kOutPieces; r < rows; r += 32 / kOutPieces)
     {
-        const int r = it * (32 / kOutPieces) + lane / kOutPieces;
-        const int m = m_base + r;
-        const int n = n_group + p * 16;
-        if (p * 16 < ncols_group && m < tp.M && n < tp.N)
+        if (p * 16 < n)
         {
-            const uint4   val = *reinterpret_cast<const uint4 *>(stage + r * kOutRowBytes + ((p ^ stage_sw(r, tma)) << 4));
-            const int64_t off = dst_off + static_cast<int64_t>(m) * tp.ldd + n;
-            if (n + 16 <= tp.N && tp.vec_ok)
+            const uint4 val = *reinterpret_cast<const uint4 *>(stage + r * kOutRowBytes + ((p ^ stage_sw(r, tma)) << 4));
+            uint8_t    *d   = d0 + r * ldd + p * 16;
+            if (p * 16 + 16 <= n)
             {
-                *reinterpret_cast<uint4 *>(tp.dst + off) = val;
-                for (int x = 0; x < tp.n_extra; ++x)
-                {
-                    *reinterpret_cast<uint4 *>(tp.extra_dst[x] + off) = val;
-                }
+                *reinterpret_cast<uint4 *>(d) = val;
             }
             else
             {
                 const uint32_t w[4] = {val.x, val.y, val.z, val.w};
-                for (int j = 0; j < 16 && n + j < tp.N; ++j)
+                for (int j = 0; j < n - p * 16; ++j)
                 {
-                    const uint8_t b    = static_cast<uint8_t>(w[j >> 2] >> (8 * (j & 3)));
-                    tp.dst[off + j]    = b;
-                    for (int x = 0; x < tp.n_extra; ++x)
-                    {
-                        tp.extra_dst[x][off + j] = b;
-                    }
+                    d[j] = static_cast<uint8_t>(w[j >> 2] >> (8 * (j & 3)));
                 }
             }
         }
     }
     __syncwarp();
+}
+
+// The same for rows that are not 16-byte aligned (N or the pitch odd): a row of the stage leaves as aligned 32-bit words,
+// shifted into place, with at most three single bytes at either end.  Per-lane byte stores wrote one byte of each of 32
+// rows per instruction, a sector each.
+// A call of its own: inlined, its addresses cost the drain of aligned rows registers.
+// d0: first valid byte of row 0 in global memory; rows, n: valid rows and bytes per row (<= 32 x kOutRowBytes).
+__device__ __noinline__ void flush_stage_words(const uint8_t *__restrict__ stage, uint8_t *__restrict__ d0, int64_t ldd, int rows, int n,
+                                               int lane)
+{
+    constexpr int kAhead = 4; // steps in flight
+    const int     shift = n <= 32 ? 3 : (n <= 64 ? 4 : 5); // lanes per row: 8, 16 or 32; the other lanes take further rows
+    const int     i = lane & ((1 << shift) - 1), kRows = 32 >> shift;
+    __syncwarp();
+#pragma unroll 1
+    for (int r0 = lane >> shift; r0 < rows; r0 += kAhead * kRows)
+    {
+        uint32_t v[kAhead], edge[kAhead]; // the lane's word; its byte at the front (lanes 0 .. 2) or at the back (4 .. 6)
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+        {
+            const int      r    = min(r0 + u * kRows, rows - 1);
+            const uint8_t *row  = stage + r * kOutRowBytes;
+            const int      sw   = stage_sw(r, false);
+            auto           word = [&](int w) { return *reinterpret_cast<const uint32_t *>(row + (((w >> 2) ^ sw) << 4) + 4 * (w & 3)); };
+            const int      head = min(n, static_cast<int>((4 - (reinterpret_cast<uintptr_t>(d0 + r * ldd) & 3)) & 3));
+            const int      tail = head + ((n - head) & ~3);
+            const uint32_t lo = word(i), hi = word(min(i + 1, kOutRowBytes / 4 - 1));
+            v[u]              = __funnelshift_r(lo, hi, 8 * head);
+            const int b       = i < 4 ? i : min(tail + i - 4, kOutRowBytes - 1);
+            edge[u]           = row[(((b >> 4) ^ sw) << 4) + (b & 15)];
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+        {
+            const int r = r0 + u * kRows;
+            if (r < rows)
+            {
+                uint8_t  *d    = d0 + r * ldd;
+                const int head = min(n, static_cast<int>((4 - (reinterpret_cast<uintptr_t>(d) & 3)) & 3));
+                const int tail = head + ((n - head) & ~3);
+                if (head + 4 * i < tail) *reinterpret_cast<uint32_t *>(d + head + 4 * i) = v[u];
+                if (i < head) d[i] = static_cast<uint8_t>(edge[u]);
+                if (i >= 4 && i < 8 && tail + i - 4 < n) d[tail + i - 4] = static_cast<uint8_t>(edge[u]);
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// 32-bit results, rows that are not 16-byte aligned: a staged chunk of 32 rows x 32 columns (128-byte swizzle) leaves as 32
+// consecutive words per row, one per lane.  o: this lane's column in row 0.
+__device__ __noinline__ void flush_raw_rows(const uint8_t *__restrict__ stage, uint8_t *__restrict__ o, int64_t ldd, int rows, int lane, EpilogueParams rp)
+{
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r)
+    {
+        const uint32_t w = *reinterpret_cast<const uint32_t *>(stage + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
+        uint32_t      *p = reinterpret_cast<uint32_t *>(o + r * ldd);
+        *p = raw_result_word(static_cast<int32_t>(w), rp.accumulate != 0 ? *p : 0u, rp);
+    }
 }
 
 // The same staged group (32 rows x kOutRowBytes, all of it valid) handed to the TMA unit: one bulk tensor store per
@@ -932,14 +983,47 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
     uint8_t      *drow    = tp.dst + row_off;
     // omap: the warp's 32 rows x kOutRowBytes leave as one bulk tensor store from its staging area (one destination)
     const bool    tma     = !kS32Out && omap != nullptr && tp.n_extra == 0; // warp-uniform
-    const bool    staged  = !kS32Out && (tp.n_extra > 0 || tma);            // warp-uniform
+    // builds of up to eight warps: everything leaves through the stage
+    const bool    staged  = !kS32Out && (kEpiWarps <= 8 || tp.n_extra > 0 || tma); // warp-uniform
     // chunk c of the warp's columns into the stage; the group goes out when it is complete
     // 32-bit results: a chunk of 32 rows x 128 bytes leaves as one bulk tensor store as well.  A lane's own stores are
     // 16-byte pieces of one row each, a row pitch apart: eight times the load/store passes, and half a sector each.
     const bool    raw_tma = kS32Out && omap != nullptr; // warp-uniform (encode_raw_map: one destination, no accumulation)
+    // Anything else (accumulation, several destinations, rows that are not 16-byte aligned) goes through the stage too and
+    // leaves as 32 consecutive words per row, one per lane.
+    const bool    raw_rows = kS32Out && kEpiWarps <= 8 && !raw_tma;
+    auto raw_rows_flush = [&](const uint32_t *v, int c) {
+        const int n = n_first + c * 32 + lane;
+        uint8_t  *row = stage + lane * 128;
+        __syncwarp();
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+        {
+            *reinterpret_cast<uint4 *>(row + ((p ^ (lane & 7)) << 4)) = make_uint4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]);
+        }
+        __syncwarp();
+        EpilogueParams rp{};
+        rp.out_f32    = tp.raw_f32;
+        rp.accumulate = tp.raw_accumulate;
+        rp.dq_scale   = tp.raw_scale;
+        const int rows = min(32, tp.M - (m - lane));
+        if (n < tp.N)
+        {
+            const int64_t off = row_off - lane * tp.ldd + 4 * static_cast<int64_t>(n);
+            for (int x = -1; x < tp.n_extra; ++x)
+            {
+                flush_raw_rows(stage, (x < 0 ? tp.dst : tp.extra_dst[x]) + off, tp.ldd, rows, lane, rp);
+            }
+        }
+    };
     auto raw_stage_and_flush = [&](const uint32_t *v, int c) {
         if (n_first + c * 32 >= tp.N)
         {
+            return;
+        }
+        if (raw_rows)
+        {
+            raw_rows_flush(v, c);
             return;
         }
         stage_reuse_wait(lane);
@@ -984,7 +1068,21 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
             }
             else
             {
-                flush_stage(stage, tp, m - lane, n_first + first * 32, ncols, lane, tma, dst_off);
+                const int rows = min(32, tp.M - (m - lane)), cols = min(ncols, tp.N - n_group);
+                if (rows > 0 && cols > 0)
+                {
+                    const int64_t off = row_off - lane * tp.ldd + n_group;
+                    for (int x = -1; x < tp.n_extra; ++x)
+                    {
+                        uint8_t *d0 = (x < 0 ? tp.dst : tp.extra_dst[x]) + off;
+                        if (tp.vec_ok != 0) flush_stage(stage, d0, tp.ldd, rows, cols, lane, tma);
+                        else flush_stage_words(stage, d0, tp.ldd, rows, cols, lane);
+                    }
+                }
+                else
+                {
+                    __syncwarp();
+                }
             }
         }
     };
@@ -1012,7 +1110,7 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
             load_residual(res, tp.residual + row_off, n_first + ch * 32, row_ok, tp);
             add_residual(va, res, tp);
         }
-        if (raw_tma)
+        if (raw_tma || raw_rows)
         {
             raw_stage_and_flush(va, ch);
         }
@@ -1046,7 +1144,7 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
                 load_residual(res, tp.residual + row_off, n_first + (ch + 1) * 32, row_ok, tp);
                 add_residual(vb, res, tp);
             }
-            if (raw_tma)
+            if (raw_tma || raw_rows)
             {
                 raw_stage_and_flush(vb, ch + 1);
             }

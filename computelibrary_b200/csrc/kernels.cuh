@@ -187,11 +187,11 @@ inline bool use_dependent_launch(const cugl_context *ctx)
 // Launch with programmatic stream serialization (griddepcontrol in the kernel): the kernel may start its prologue while the
 // previous kernel of the stream is finishing.  ctx->dependent_launch == 0 or a capturing stream: a plain launch.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent_cluster(cugl_context *ctx, void (*kernel)(KArgs...), int grid, int threads, int smem_bytes, int cluster,
+cudaError_t launch_dependent_cluster(cugl_context *ctx, void (*kernel)(KArgs...), dim3 grid, int threads, int smem_bytes, int cluster,
                                      Args &&...args)
 {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim          = dim3(static_cast<unsigned>(grid), 1, 1);
+    cfg.gridDim          = grid;
     cfg.blockDim         = dim3(static_cast<unsigned>(threads), 1, 1);
     cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
     cfg.stream           = ctx->stream;
@@ -216,7 +216,7 @@ cudaError_t launch_dependent_cluster(cugl_context *ctx, void (*kernel)(KArgs...)
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(cugl_context *ctx, void (*kernel)(KArgs...), int grid, int threads, int smem_bytes, Args &&...args)
+cudaError_t launch_dependent(cugl_context *ctx, void (*kernel)(KArgs...), dim3 grid, int threads, int smem_bytes, Args &&...args)
 {
     return launch_dependent_cluster(ctx, kernel, grid, threads, smem_bytes, 1, static_cast<Args &&>(args)...);
 }
