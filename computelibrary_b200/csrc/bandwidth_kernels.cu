@@ -176,7 +176,7 @@ struct PrepParams
 {
     OperandPrep op;
     int         b_strips, b_splits, b_blocks, k_per_split; // strips of 64 columns, K splits of k_per_split rows
-    int         row_lanes; // lanes that share a row of A
+    int         row_lanes; // lanes that share a row of A (kThreads: a block each)
     bool        b_words, a_vec; // B rows 4-byte aligned / A rows 16-byte aligned
 };
 
@@ -309,6 +309,37 @@ __device__ __forceinline__ uint4 load_row16(const uint8_t *row, int k, int K, bo
     return make_uint4(v[0], v[1], v[2], v[3]);
 }
 
+// Few long rows: a block per row, so that no warp walks a whole row alone (16 rows of 5429 bytes: eleven steps of 512).
+__device__ __forceinline__ void prepare_a_row_blocks(const PrepParams &p, int block, int32_t *partial)
+{
+    const OperandPrep &o   = p.op;
+    const int64_t      m   = block;
+    const int64_t      z   = o.batch_a > 1 ? m / o.rows : 0;
+    const uint8_t     *row = o.a + z * o.a_batch_stride + (m - z * o.rows) * o.lda;
+    uint8_t           *out = o.copy != nullptr ? o.copy + m * o.kp : nullptr;
+    int32_t            acc = 0;
+    for (int k = 16 * static_cast<int>(threadIdx.x); k < o.K; k += 16 * kThreads)
+    {
+        const uint4 v = load_row16(row, k, o.K, p.a_vec);
+        if (out != nullptr) *reinterpret_cast<uint4 *>(out + k) = v;
+        acc = sum4(v.x, o.a_signed, acc);
+        acc = sum4(v.y, o.a_signed, acc);
+        acc = sum4(v.z, o.a_signed, acc);
+        acc = sum4(v.w, o.a_signed, acc);
+    }
+    if (o.rowsum != nullptr)
+    {
+        acc = warp_sum(acc);
+        if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            for (int w = 1; w < kThreads / 32; ++w) acc += partial[w];
+            o.rowsum[m] = acc;
+        }
+    }
+}
+
 __device__ __forceinline__ void prepare_a_rows(const PrepParams &p, int block, int n_blocks)
 {
     const OperandPrep &o    = p.op;
@@ -372,6 +403,10 @@ __global__ void __launch_bounds__(kThreads) prepare_operands_kernel(const __grid
     if (block < p.b_blocks)
     {
         prepare_b_strip(p, block, tile);
+    }
+    else if (p.row_lanes == kThreads)
+    {
+        prepare_a_row_blocks(p, block - p.b_blocks, reinterpret_cast<int32_t *>(tile));
     }
     else
     {
@@ -810,6 +845,13 @@ cugl_status launch_prepare_operands(cugl_context *ctx, const OperandPrep &op)
         p.row_lanes = 1;
         while (p.row_lanes < 32 && p.row_lanes * 16 < op.K) p.row_lanes *= 2;
         a_blocks = grid_for(static_cast<int64_t>(op.rows) * op.batch_a * p.row_lanes, ctx->sm_count);
+        // rows of more than one step per warp, and at most two blocks per SM if every row gets its own
+        const int64_t all_rows = static_cast<int64_t>(op.rows) * op.batch_a;
+        if (op.K > 512 && op.fill == 0 && all_rows <= 2 * ctx->sm_count)
+        {
+            p.row_lanes = kThreads;
+            a_blocks    = static_cast<int>(all_rows);
+        }
     }
     if (p.b_blocks + a_blocks == 0) return CUGL_SUCCESS;
     CUGL_CUDA_TRY(ctx, launch_dependent(ctx, prepare_operands_kernel, p.b_blocks + a_blocks, kThreads, 0, p));
