@@ -395,10 +395,7 @@ __device__ __forceinline__ void prepare_a_rows(const PrepParams &p, int block, i
 __global__ void __launch_bounds__(kThreads) prepare_operands_kernel(const __grid_constant__ PrepParams p)
 {
     __shared__ uint32_t tile[64][33];
-    // the tensor-core kernel behind this launch may set itself up meanwhile; this kernel itself touches memory only
-    // after everything before it in the stream has completed
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    dependent_prologue(); // the tensor-core kernel behind this launch sets itself up meanwhile
     const int block = static_cast<int>(blockIdx.x);
     if (block < p.b_blocks)
     {
@@ -492,9 +489,7 @@ __global__ void __launch_bounds__(kThreads) output_stage_kernel(const int32_t *_
                                                                 int32_t shift, int32_t offset, int32_t lo, int32_t hi,
                                                                 bool vec_ok, bool integer_stage)
 {
-    // behind the product that writes its input: scheduled while that kernel finishes, no access before it has
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    dependent_prologue(); // behind the product that writes its input
     const int n0 = (blockIdx.x * kThreads + threadIdx.x) * 4;
     if (n0 >= N)
     {
@@ -663,6 +658,7 @@ template <bool kFast>
 __global__ void __launch_bounds__(kThreads) fold_input_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
                                                               int B, int H, int W, int C, int H2, int W2, uint32_t zp)
 {
+    dependent_prologue();
     const int64_t total = static_cast<int64_t>(B) * H2 * W2;
     for (int64_t i = blockIdx.x * static_cast<int64_t>(kThreads) + threadIdx.x; i < total;
          i += static_cast<int64_t>(gridDim.x) * kThreads)
@@ -854,7 +850,7 @@ cugl_status launch_prepare_operands(cugl_context *ctx, const OperandPrep &op)
         }
     }
     if (p.b_blocks + a_blocks == 0) return CUGL_SUCCESS;
-    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, prepare_operands_kernel, p.b_blocks + a_blocks, kThreads, 0, p));
+    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, prepare_operands_kernel, p.b_blocks + a_blocks, kThreads, 0, p.b_blocks + a_blocks, p));
     return check_cuda(ctx, cudaGetLastError(), "prepare_operands_kernel");
 }
 
@@ -911,13 +907,13 @@ cugl_status launch_output_stage(cugl_context *ctx, const int32_t *d_in, int64_t 
     const dim3 blocks(gx, gy);
     if (out16)
     {
-        CUGL_CUDA_TRY(ctx, launch_dependent(ctx, output_stage_kernel<true>, blocks, kThreads, 0,
+        CUGL_CUDA_TRY(ctx, launch_dependent(ctx, output_stage_kernel<true>, blocks, kThreads, 0, gx * gy,
             d_in, ld_in_bytes / 4, d_bias, static_cast<uint8_t *>(d_out), ld_out_bytes, M, N, d_mults, d_shifts, mult,
             shift, offset, lo, hi, vec_ok, integer_stage));
     }
     else
     {
-        CUGL_CUDA_TRY(ctx, launch_dependent(ctx, output_stage_kernel<false>, blocks, kThreads, 0,
+        CUGL_CUDA_TRY(ctx, launch_dependent(ctx, output_stage_kernel<false>, blocks, kThreads, 0, gx * gy,
             d_in, ld_in_bytes / 4, d_bias, static_cast<uint8_t *>(d_out), ld_out_bytes, M, N, d_mults, d_shifts, mult,
             shift, offset, lo, hi, vec_ok, integer_stage));
     }
@@ -980,15 +976,13 @@ cugl_status launch_fold_input(cugl_context *ctx, const void *d_src, void *d_dst,
                       static_cast<int64_t>(B) * H2 * W2 <= 0x7fffffff;
     if (fast)
     {
-        fold_input_kernel<true><<<blocks, kThreads, 0, ctx->stream>>>(static_cast<const uint8_t *>(d_src),
-                                                                      static_cast<uint8_t *>(d_dst), B, H, W, C, H2, W2,
-                                                                      static_cast<uint32_t>(zero_point) & 0xffu);
+        CUGL_CUDA_TRY(ctx, launch_blocks(ctx, fold_input_kernel<true>, blocks, static_cast<const uint8_t *>(d_src),
+                                            static_cast<uint8_t *>(d_dst), B, H, W, C, H2, W2, static_cast<uint32_t>(zero_point) & 0xffu));
     }
     else
     {
-        fold_input_kernel<false><<<blocks, kThreads, 0, ctx->stream>>>(static_cast<const uint8_t *>(d_src),
-                                                                       static_cast<uint8_t *>(d_dst), B, H, W, C, H2, W2,
-                                                                       static_cast<uint32_t>(zero_point) & 0xffu);
+        CUGL_CUDA_TRY(ctx, launch_blocks(ctx, fold_input_kernel<false>, blocks, static_cast<const uint8_t *>(d_src),
+                                            static_cast<uint8_t *>(d_dst), B, H, W, C, H2, W2, static_cast<uint32_t>(zero_point) & 0xffu));
     }
     return check_cuda(ctx, cudaGetLastError(), "fold_input_kernel");
 }

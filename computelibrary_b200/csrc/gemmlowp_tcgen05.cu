@@ -3635,7 +3635,7 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
     {
         tp.pair_drain = 0;
     }
-    CUGL_CUDA_TRY(ctx, launch_dependent_cluster(ctx, kernel, grid, kThreads, kDynBytes, kSplit ? op.split_k : 1, map_a, map_b, map_out, map_res, tp, ep));
+    CUGL_CUDA_TRY(ctx, launch_dependent_cluster(ctx, kernel, grid, kThreads, kDynBytes, kSplit ? op.split_k : 1, units, map_a, map_b, map_out, map_res, tp, ep));
     return check_cuda(ctx, cudaGetLastError(), "gemmlowp_tcgen05_kernel");
 }
 
@@ -3681,7 +3681,7 @@ cugl_status launch_variant_cm(cugl_context *ctx, const GemmOperands &op, const E
     tp.split_tail = 0;
     const int tiles = ((op.N + BLOCK_M - 1) / BLOCK_M) * ((op.M + BLOCK_N - 1) / BLOCK_N);
     const int grid  = tiles < ctx->sm_count ? tiles : ctx->sm_count;
-    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, kernel, grid, kThreads, P::DYN_BYTES, map_w, map_x, map_w, map_w, tp, ep)); // (no bulk stores on this path)
+    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, kernel, grid, kThreads, P::DYN_BYTES, tiles, map_w, map_x, map_w, map_w, tp, ep)); // (no bulk stores on this path)
     return check_cuda(ctx, cudaGetLastError(), "gemmlowp_tcgen05_kernel (channel-major)");
 }
 
@@ -3741,22 +3741,9 @@ cugl_status launch_variant_2cta(cugl_context *ctx, const GemmOperands &op, const
     const int pairs    = ctx->sm_count / 2;
     const int clusters = tiles < pairs ? tiles : pairs;
 
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim          = dim3(2 * clusters, 1, 1);
-    cfg.blockDim         = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = P::DYN_BYTES;
-    cfg.stream           = ctx->stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id               = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id               = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs                = attr;
-    cfg.numAttrs             = use_dependent_launch(ctx) ? 2 : 1;
     tp.tma_store = tma_store ? 1 : 0;
-    CUGL_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_bh, map_out, tp, ep));
+    CUGL_CUDA_TRY(ctx, launch_dependent_cluster(ctx, kernel, 2 * clusters, kThreads, P::DYN_BYTES, 2, 2ll * tiles, map_a, map_b, map_bh,
+                                                map_out, tp, ep));
     return CUGL_SUCCESS;
 }
 
@@ -3831,7 +3818,7 @@ cugl_status launch_conv_variant(cugl_context *ctx, const GemmOperands &op, const
     const int tiles = ((op.M + MT * BLOCK_M - 1) / (MT * BLOCK_M)) * ((op.N + BLOCK_N - 1) / BLOCK_N); // units of MT tiles
     const int grid  = tiles < ctx->sm_count ? tiles : ctx->sm_count;
     tp.tma_store = tma_store ? 1 : 0;
-    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, kernel, grid, kConvThreads, kDynBytes, map_b, map_out, tp, ep, cg));
+    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, kernel, grid, kConvThreads, kDynBytes, tiles, map_b, map_out, tp, ep, cg));
     return check_cuda(ctx, cudaGetLastError(), "gemmlowp_conv_tcgen05_kernel");
 }
 #endif // CUGL_TC_FULL_BUILD

@@ -167,9 +167,12 @@ bool classify_add(float a_scale, int a_zp, float b_scale, int b_zp, float o_scal
                   float act_b, int *floor_out, int *cap_out);
 
 // Programmatic stream serialization pays where launches are issued one by one (QASYMM8 ResNet-50, batch 256, layer
-// by layer: 2.74 -> 2.67 ms); inside a captured graph, whose launches are packed already, the programmatic edges
-// measured 1 % slower (2.594 -> 2.618 ms), so a capturing stream gets plain launches.
-inline bool use_dependent_launch(const cugl_context *ctx)
+// by layer: 2.74 -> 2.67 ms).  Inside a captured graph, whose launches are packed already, it pays for short launches, whose
+// set-up is a good part of them, and costs for long ones (ResNet-50 as a graph without / with programmatic edges
+// everywhere: batch 1 385 / 365 us, 4 452 / 428, 16 602 / 589, 64 1026 / 1013, 256 2604 / 2621): a capturing stream
+// gets it where the launch has at most kShortWaves units of work per SM.
+constexpr int kShortWaves = 4;
+inline bool use_dependent_launch(const cugl_context *ctx, long long units)
 {
     if (ctx->dependent_launch == 0)
     {
@@ -181,14 +184,22 @@ inline bool use_dependent_launch(const cugl_context *ctx)
         (void)cudaGetLastError();
         return false;
     }
-    return st == cudaStreamCaptureStatusNone;
+    return st == cudaStreamCaptureStatusNone || units <= static_cast<long long>(kShortWaves) * ctx->sm_count;
+}
+
+// First thing in a kernel launched with launch_dependent that has no prologue worth overlapping: the next kernel of the
+// stream may set itself up, this one touches memory only after everything before it has completed.
+__device__ __forceinline__ void dependent_prologue()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Launch with programmatic stream serialization (griddepcontrol in the kernel): the kernel may start its prologue while the
-// previous kernel of the stream is finishing.  ctx->dependent_launch == 0 or a capturing stream: a plain launch.
+// previous kernel of the stream is finishing.  units: tiles or blocks of work in the launch (use_dependent_launch).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dependent_cluster(cugl_context *ctx, void (*kernel)(KArgs...), dim3 grid, int threads, int smem_bytes, int cluster,
-                                     Args &&...args)
+                                     long long units, Args &&...args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim          = grid;
@@ -205,7 +216,7 @@ cudaError_t launch_dependent_cluster(cugl_context *ctx, void (*kernel)(KArgs...)
         attr[n].val.clusterDim.z = 1;
         ++n;
     }
-    if (use_dependent_launch(ctx))
+    if (use_dependent_launch(ctx, units))
     {
         attr[n].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
@@ -216,8 +227,22 @@ cudaError_t launch_dependent_cluster(cugl_context *ctx, void (*kernel)(KArgs...)
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(cugl_context *ctx, void (*kernel)(KArgs...), dim3 grid, int threads, int smem_bytes, Args &&...args)
+cudaError_t launch_dependent(cugl_context *ctx, void (*kernel)(KArgs...), dim3 grid, int threads, int smem_bytes, long long units, Args &&...args)
 {
-    return launch_dependent_cluster(ctx, kernel, grid, threads, smem_bytes, 1, static_cast<Args &&>(args)...);
+    return launch_dependent_cluster(ctx, kernel, grid, threads, smem_bytes, 1, units, static_cast<Args &&>(args)...);
+}
+// The byte kernels between the products: blocks of 256 threads, dependent only where the launch is short (a network at
+// batch 1; with several blocks of work per SM the waiting successor's blocks are in the way, 256 global averages of
+// 7 x 7 x 2048: 12.3 against 14.8 us).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_blocks(cugl_context *ctx, void (*kernel)(KArgs...), int blocks, Args &&...args)
+{
+    const bool short_launch = blocks <= ctx->sm_count;
+    if (!short_launch)
+    {
+        kernel<<<blocks, 256, 0, ctx->stream>>>(static_cast<KArgs>(args)...);
+        return cudaGetLastError();
+    }
+    return launch_dependent(ctx, kernel, blocks, 256, 0, blocks, static_cast<Args &&>(args)...);
 }
 } // namespace cugl
