@@ -151,9 +151,11 @@ cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, c
     // sixteen epilogue warps (256-column tiles only) buy another 4 - 7 % on short K with wide outputs
     // (up to K = 512, where its paired drain applies; above, eight warps -- whose single-tile drain stores through the
     // TMA unit -- measured faster: 50176 x 256 x 1024 25.5 against 27.6 us)
-    // Also for rows of dst that are not 16-byte aligned, although only the smaller builds stage those: 4000 x 5001 x 512
-    // 28.2 us against 36.5 with eight warps.
-    if (o.N > 128 && (o.epi_warps == 16 || (ep.stage != CUGL_STAGE_NONE && o.epi_warps != 4 && o.epi_warps != 8 && o.K <= 512)))
+    // Rows of dst that are not 16-byte aligned: only the smaller builds stage those, the sixteen-warp row-major drain writes
+    // them byte by byte (2099 x 3709 x 352: 91 us against 21 with eight warps, 8000 x 1001 x 64: 87 / 20); channel-major
+    // keeps its sixteen (4000 x 5001 x 512: 28 / 37).
+    const bool dst_rows = ((reinterpret_cast<uintptr_t>(o.dst) | static_cast<uint64_t>(o.ldd)) & 15) == 0;
+    if (o.N > 128 && (o.epi_warps == 16 || ((dst_rows || o.channel_major > 0) && ep.stage != CUGL_STAGE_NONE && o.epi_warps != 4 && o.epi_warps != 8 && o.K <= 512)))
     {
         return launch_gemmlowp_tcgen05_epi16(ctx, o, ep, false);
     }
