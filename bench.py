@@ -857,7 +857,7 @@ def run_bandwidth(args):
     desc, keep = capi.make_gemm_desc(128, N, K, capi.S8, capi.S8, capi.S8, 5, 0, multiplier=2 ** 30, shift=8,
                                      min_bound=-128, max_bound=127)
     plan, b = capi.GemmPlan(ctx, desc, keep), rnd8(K, N)
-    case("transpose_colsum_kernel", 2 * K * N + 4 * N, lambda: plan.prepare(b), f"B s8 [{K}][{N}] -> Bt + column sums")
+    case("prepare_operands_kernel", 2 * K * N + 4 * N, lambda: plan.prepare(b), f"B s8 [{K}][{N}] -> Bt + column sums")
     plan.close()
     del b
     M, N = 8192 // sc, 8192
