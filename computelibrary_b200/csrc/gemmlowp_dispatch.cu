@@ -77,6 +77,19 @@ int pick_split(const cugl_context *ctx, const GemmOperands &op)
     return 1;
 }
 
+// 8-bit rows of dst that are not 16-byte aligned cannot leave as bulk tensor stores.  The channel-major kernel with sixteen
+// warps, whose lanes write eight neighbouring rows' bytes of their channel, is the fastest way out for them wherever its
+// 128-channel x 256-row tiles occupy half the device; against the row-major kernel's staged words (eight warps), us:
+// 2099 x 3709 x 352 13.5 / 20.7, 4000 x 5001 x 64 26.8 / 45.3, x 1000 39.7 / 54.7, 8000 x 301 x 256 8.4 / 11.8,
+// 500 x 6001 x 352 8.8 / 12.1.  Longer K belongs to the main loop and to the SM pair.
+bool ragged_rows_channel_major(const cugl_context *ctx, const GemmOperands &op)
+{
+    const bool      aligned = ((reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd)) & 15) == 0;
+    const long long tiles   = static_cast<long long>((op.N + 127) / 128) * ((op.M + 255) / 256);
+    return !aligned && op.channel_major == 0 && op.epi_warps == 0 && op.block_n == 0 && op.batch <= 1 && op.n_extra_dst == 0 &&
+           op.conv == nullptr && op.K <= kShortK && tiles >= ctx->sm_count / 2;
+}
+
 // the SM-pair kernel works on 256 x 256 tiles, one per pair of SMs
 bool pair_fills_the_device(const cugl_context *ctx, const GemmOperands &op)
 {
@@ -117,6 +130,11 @@ cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, c
         o.split_k       = split;
         o.channel_major = -1;
         return launch_gemmlowp_tcgen05_epi8(ctx, o, ep, false);
+    }
+    if (ep.stage != CUGL_STAGE_NONE && ep.rowsum == nullptr && ragged_rows_channel_major(ctx, op))
+    {
+        o.channel_major = 1;
+        return launch_gemmlowp_tcgen05_epi16(ctx, o, ep, false);
     }
     o.block_n        = pick_block_n(ctx, op); // before the automatic channel-major choice below
     if (op.batch > 1)

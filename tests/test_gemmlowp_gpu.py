@@ -221,6 +221,22 @@ def test_32_bit_results_through_bulk_stores(ctx, port, M, N, K, ldd_pad):
         assert np.array_equal(f, core.astype(np.float32) * np.float32(1.3e-4)), store
 
 
+@pytest.mark.parametrize("M,N,K,ldd_pad", [(300, 9601, 64, 0), (257, 5001, 200, 0), (2400, 1001, 130, 3), (2432, 1024, 1024, 5),
+                                           (2400, 1001, 1025, 0), (9700, 129, 16, 2)])
+def test_ragged_output_rows(ctx, port, M, N, K, ldd_pad):
+    """8-bit rows that are not 16-byte aligned: the channel-major kernel inside its rule, the staged words just outside it
+    (K = 1025), canary bytes around every row, per-channel stages of both output types."""
+    rng = np.random.default_rng(M + N + K)
+    for t, a_off in ((np.uint8, -128), (np.int8, 5)):
+        a, b = q8_uniform(rng, (M, K), t), q8_uniform(rng, (K, N), np.int8, -127, 127)
+        lo, hi = type_range(t)
+        bias = rng.integers(-2000, 2001, N).astype(np.int32)
+        mult = rng.integers(2 ** 30, 2 ** 31 - 1, N).astype(np.int32)
+        shift = rng.integers(8, 14, N).astype(np.int32)
+        got, _ = gpu_gemmlowp(ctx, a, b, bias, a_off, 0, mult, shift, 3, lo, hi, t, ldd_pad=ldd_pad)
+        assert np.array_equal(got, port.gemmlowp_fused(a, b, bias, a_off, 0, mult, shift, 3, lo, hi, t)), t
+
+
 def test_run_twice_and_variable_b(ctx, port):
     """MultipleExecution (GEMMLowp.cpp:211-297): same plan, same output; B re-laid out per run when it is
     not constant (reshape_b_only_on_first_run = false)."""
