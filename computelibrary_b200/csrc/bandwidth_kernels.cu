@@ -812,12 +812,14 @@ cugl_status launch_prepare_operands(cugl_context *ctx, const OperandPrep &op)
     p.op = op;
     if (op.b != nullptr && op.N > 0 && op.K > 0)
     {
-        // One strip of 64 columns per block, all of K, when the strips alone give every SM a block: the column sums then
-        // need neither zeroed memory nor atomics.  Else K is split until about two blocks per SM exist.
+        // One strip of 64 columns per block, all of K, when K is short or the strips alone give every SM six blocks: the column
+        // sums then need neither zeroed memory nor atomics.  Else K is split until about six blocks per SM exist: a block
+        // waits for one tile's loads at a time (4096 x 14336: a block per strip 67 us, six blocks per SM 41; 4096 x 4096: two
+        // blocks per SM 12.6, six 10.5).
         p.b_strips = (op.N + 63) / 64;
         const int64_t strips = static_cast<int64_t>(p.b_strips) * op.batch_b;
         const int64_t k_tiles = (op.K + 127) / 128;
-        int64_t splits = strips >= ctx->sm_count ? 1 : (2 * ctx->sm_count + strips - 1) / strips;
+        int64_t splits = strips >= 6 * ctx->sm_count ? 1 : (6 * ctx->sm_count + strips - 1) / strips;
         splits         = splits < k_tiles ? splits : k_tiles;
         if (k_tiles <= 4) splits = 1; // a strip of a few tiles is finished sooner than a memset and its launch
         const int64_t tiles_per_split = (k_tiles + splits - 1) / splits;
