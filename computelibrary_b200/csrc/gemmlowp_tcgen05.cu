@@ -60,6 +60,8 @@ static_assert(kEpiWarps == 4 || kEpiWarps == 8 || kEpiWarps == 16, "epilogue war
 // The sixteen-warp build holds only the one-CTA GEMM kernels with 256-column tiles (row-major and channel-major):
 // the kernels for short K and wide outputs, whose epilogue wants the most latency hiding.
 #define CUGL_TC_FULL_BUILD (CUGL_EPI_WARPS <= 8)
+// The SM-pair kernel belongs to the four-warp build: it serves long K, where extra epilogue warps only slow the main loop.
+#define CUGL_TC_PAIR_BUILD (CUGL_EPI_WARPS == 4)
 constexpr int      A_STAGE     = BLOCK_M * BLOCK_K;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
@@ -2505,7 +2507,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 
-#if CUGL_TC_FULL_BUILD
+#if CUGL_TC_PAIR_BUILD
 // ---------------------------------------------------------------------------------------------------
 // Two-CTA kernel: a cluster of two CTAs (an SM pair) per 256 x 256 output tile.
 //   CTA rank r stages rows [m0 + 128 r, +128) of A and rows [n0 + 128 r, +128) of Bt (its half of the
@@ -2513,7 +2515,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 //   the epilogue for them.  The MMA issuer of rank 0 drives the tensor cores of both SMs.
 //   Barriers: full[] lives in rank 0 and collects the bytes of both CTAs' copies; empty[] and tfull[]
 //   exist in both CTAs and are signalled together by a multicast tcgen05.commit; tempty[] lives in rank 0
-//   and is arrived on by the sixteen epilogue warps of the pair.
+//   and is arrived on by the epilogue warps of both CTAs.
 // ---------------------------------------------------------------------------------------------------
 template <int STAGES, int KSUB>
 struct SmemPlan2
@@ -2543,6 +2545,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 {
     using P               = SmemPlan2<STAGES, KSUB>;
     constexpr int BLOCK_N = P::BLOCK_N;
+    static_assert(!kS32Out || kOutStageBytes >= kRawStageBytes, "a warp stages 32-bit results in kRawStageBytes of shared memory");
     extern __shared__ uint8_t smem_raw[];
     // the 1024-byte aligned start of the dynamic shared memory, derived by pointer arithmetic on the __shared__ array
     // itself: a pointer rebuilt from an integer loses its address space and every access through it becomes a
@@ -2877,8 +2880,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         atomicCAS(tp.status, 0, *s_abort);
     }
 }
+#endif // CUGL_TC_PAIR_BUILD
 
-
+#if CUGL_TC_FULL_BUILD
 // ---------------------------------------------------------------------------------------------------
 // Implicit-GEMM convolution (NHWC, 8-bit): the same one-CTA pipeline, but the A tile (128 output pixels x
 // 128 bytes of the (ky, kx, c) patch axis) is gathered straight from the input tensor by four extra warps
@@ -3685,7 +3689,7 @@ cugl_status launch_variant_cm(cugl_context *ctx, const GemmOperands &op, const E
     return check_cuda(ctx, cudaGetLastError(), "gemmlowp_tcgen05_kernel (channel-major)");
 }
 
-#if CUGL_TC_FULL_BUILD
+#if CUGL_TC_PAIR_BUILD
 template <int STAGES, int KSUB, bool kS32Out>
 cugl_status launch_variant_2cta(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
 {
@@ -3705,7 +3709,7 @@ cugl_status launch_variant_2cta(cugl_context *ctx, const GemmOperands &op, const
     {
         return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the output tiles");
     }
-    if (kS32Out && kEpiWarps == 4 && !encode_raw_map(op, ep, &map_out, &tma_store)) // (four warps: their staging has the size)
+    if (kS32Out && !encode_raw_map(op, ep, &map_out, &tma_store))
     {
         return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the output tiles");
     }
@@ -3746,7 +3750,9 @@ cugl_status launch_variant_2cta(cugl_context *ctx, const GemmOperands &op, const
                                                 map_out, tp, ep));
     return CUGL_SUCCESS;
 }
+#endif // CUGL_TC_PAIR_BUILD
 
+#if CUGL_TC_FULL_BUILD
 template <int BLOCK_N, int STAGES, int KSUB, int ACC, int RESB = 0, int MT = 1>
 cugl_status launch_conv_variant(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,
                                 const ConvOperands &cv)
@@ -3846,11 +3852,13 @@ bool CUGL_TC_NAME(gemmlowp_conv_tma_supported)(const GemmOperands &op)
     return (bits & 15) == 0 && get_encode_fn() != nullptr && conv_tma_supported(op);
 }
 
+#if CUGL_TC_PAIR_BUILD
 // The SM-pair kernel pays off once a tile spans both halves: more than 128 rows and more than 128 columns.
 bool CUGL_TC_NAME(gemmlowp_tcgen05_uses_pair)(const GemmOperands &op)
 {
     return op.N > 128 && op.M > 128;
 }
+#endif
 
 cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,
                                     bool allow_pair)
@@ -3881,7 +3889,7 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
     {
         return s32 ? launch_variant_cm<256, 4, 1, true>(ctx, op, ep) : launch_variant_cm<256, 4, 1, false>(ctx, op, ep);
     }
-#if CUGL_TC_FULL_BUILD
+#if CUGL_TC_PAIR_BUILD
     if (allow_pair && CUGL_TC_NAME(gemmlowp_tcgen05_uses_pair)(op) && !(op.conv != nullptr && op.conv->C == 64)) // (64-byte-swizzle tiles: one-CTA kernels)
     {
         return s32 ? launch_variant_2cta<3, 2, true>(ctx, op, ep) : launch_variant_2cta<3, 2, false>(ctx, op, ep);

@@ -141,7 +141,6 @@ bool        gemmlowp_conv_tma_supported_epi4(const GemmOperands &op); // op.conv
 bool        gemmlowp_conv_tma_supported(const GemmOperands &op);
 bool        gemmlowp_tcgen05_supported_epi8(const GemmOperands &op);
 bool        gemmlowp_tcgen05_uses_pair_epi4(const GemmOperands &op);
-bool        gemmlowp_tcgen05_uses_pair_epi8(const GemmOperands &op);
 cugl_status launch_gemmlowp_tcgen05_epi4(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,
                                          bool allow_pair);
 cugl_status launch_gemmlowp_tcgen05_epi8(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,
