@@ -804,8 +804,9 @@ __device__ __noinline__ void flush_stage(const uint8_t *stage, uint8_t *d0, int6
 // rows per instruction, a sector each.
 // A call of its own: inlined, its addresses cost the drain of aligned rows registers.
 // d0: first valid byte of row 0 in global memory; rows, n: valid rows and bytes per row (<= 32 x kOutRowBytes).
+// tma: the stage is in the tensor map's swizzle (dst would take bulk stores, it is the residual whose rows are not aligned).
 __device__ __noinline__ void flush_stage_words(const uint8_t *__restrict__ stage, uint8_t *__restrict__ d0, int64_t ldd, int rows, int n,
-                                               int lane)
+                                               int lane, bool tma)
 {
     constexpr int kAhead = 4; // steps in flight
     const int     shift = n <= 32 ? 3 : (n <= 64 ? 4 : 5); // lanes per row: 8, 16 or 32; the other lanes take further rows
@@ -820,7 +821,7 @@ __device__ __noinline__ void flush_stage_words(const uint8_t *__restrict__ stage
         {
             const int      r    = min(r0 + u * kRows, rows - 1);
             const uint8_t *row  = stage + r * kOutRowBytes;
-            const int      sw   = stage_sw(r, false);
+            const int      sw   = stage_sw(r, tma);
             auto           word = [&](int w) { return *reinterpret_cast<const uint32_t *>(row + (((w >> 2) ^ sw) << 4) + 4 * (w & 3)); };
             const int      head = min(n, static_cast<int>((4 - (reinterpret_cast<uintptr_t>(d0 + r * ldd) & 3)) & 3));
             const int      tail = head + ((n - head) & ~3);
@@ -1078,7 +1079,7 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
                     {
                         uint8_t *d0 = (x < 0 ? tp.dst : tp.extra_dst[x]) + off;
                         if (tp.vec_ok != 0) flush_stage(stage, d0, tp.ldd, rows, cols, lane, tma);
-                        else flush_stage_words(stage, d0, tp.ldd, rows, cols, lane);
+                        else flush_stage_words(stage, d0, tp.ldd, rows, cols, lane, tma);
                     }
                 }
                 else

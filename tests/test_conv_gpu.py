@@ -239,6 +239,43 @@ def test_fused_residual_addition(ctx, port, geom):
     plan.close()
 
 
+@pytest.mark.parametrize("H,C,OFM,k", [(7, 2048, 64, 1), (7, 2048, 48, 1), (14, 2064, 512, 1), (14, 128, 64, 3), (5, 256, 160, 3), (11, 1040, 72, 1),
+                                        (13, 1200, 64, 1)])
+def test_residual_of_any_alignment(ctx, port, H, C, OFM, k):
+    """A fused residual whose rows are not 16-byte aligned while the destination's are (and the other way round, and both):
+    layers of few tiles, whose K is shared by a cluster, and narrow tiles of the four-warp build; in place too."""
+    import torch
+    rng = np.random.default_rng(H * C + OFM)
+    src = q8_uniform(rng, (1, H, H, C), np.uint8)
+    wgt = q8_uniform(rng, (OFM, k, k, C), np.int8, -127, 127)
+    bias = rng.integers(-3000, 3001, OFM).astype(np.int32)
+    ws = (np.exp(rng.uniform(np.log(1e-3), np.log(1e-2), OFM)) / np.sqrt(k * k * C) * 8).astype(np.float32)
+    q = (0.05, 0)
+    mult, shift = f32_mults(port, q[0], ws, q[0])
+    conv = port.conv2d_nhwc(src, wgt, bias, (1, 1), (k // 2,) * 4, q[1], 0, mult, shift, q[1], 0, 255)
+    res = q8_uniform(rng, conv.shape, np.uint8)
+    want = port.activation_qasymm8(port.add_qasymm8(conv, res, q, q, q), "relu", 0.0, 0.0, q, q)
+    desc, keep = capi.make_conv_desc(1, H, H, C, OFM, k, k, (1, 1), (k // 2,) * 4, (1, 1), capi.U8, capi.S8, q[1], 0,
+                                     multipliers=mult, shifts=shift, dst_zp=q[1], min_bound=0, max_bound=255)
+    plan = capi.ConvPlan(ctx, desc, keep)
+    plan.set_residual(q[0], q, q, act=capi.ACT_RELU)
+    plan.prepare(torch.from_numpy(wgt.view(np.uint8)).cuda())
+    d_src, d_b, n = torch.from_numpy(src).cuda(), torch.from_numpy(bias).cuda(), res.size
+    for res_at, dst_at in ((0, 0), (1, 0), (8, 0), (0, 1), (3, 5), (16, 16)):
+        r_whole = torch.full((n + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+        d_whole = torch.full((n + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+        r, d = r_whole[res_at:res_at + n], d_whole[dst_at:dst_at + n]
+        r.copy_(torch.from_numpy(res.reshape(-1)))
+        plan.run_residual(d_src, d_b, r, d)
+        plan.run_residual(d_src, d_b, r, r)
+        ctx.sync()
+        for whole, at in ((d_whole, dst_at), (r_whole, res_at)):
+            everything = whole.cpu().numpy()
+            assert np.array_equal(everything[at:at + n], want.reshape(-1)), (res_at, dst_at)
+            assert (everything[:at] == 0xA5).all() and (everything[at + n:] == 0xA5).all(), (res_at, dst_at)
+    plan.close()
+
+
 @pytest.mark.parametrize("OFM", [256, 384])
 @pytest.mark.parametrize("paired", [True, False])
 def test_short_k_many_tiles_with_and_without_residual(ctx, port, paired, OFM):
