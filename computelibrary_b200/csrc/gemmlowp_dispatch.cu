@@ -90,6 +90,21 @@ bool ragged_rows_channel_major(const cugl_context *ctx, const GemmOperands &op)
            op.conv == nullptr && op.K <= kShortK && tiles >= ctx->sm_count / 2;
 }
 
+// Four or eight epilogue warps for a batch in one launch.  The batched kernels fill every wave, so that the shorter main
+// loop of four warps pays later than in single products, us with eight / four: 2 x 2432 x 2432 x 1152 18.9 / 19.6,
+// 4 x 1500^3 (ragged rows) 32 / 38, 2 x 8192 x 2048 x 1280 40.8 / 39.1, 4 x 2304 x 2304 x 1536 36.7 / 32.8,
+// 2 x 2048 x 2304 x 8192 to float32 77 / 69.  Ragged 8-bit rows leave through the staged words, which want eight warps until
+// the main loop hides them: 2 x 4000 x 5001 x 2000 99 / 127, 2 x 2500 x 2501 x 4096 55.9 / 54.8.
+bool batch_eight_epilogue_warps(const GemmOperands &op, bool output_stage)
+{
+    if (op.epi_warps == 4 || op.epi_warps == 8)
+    {
+        return op.epi_warps == 8;
+    }
+    const bool ragged = output_stage && ((reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd)) & 15) != 0;
+    return op.K < (ragged ? 4096 : 1280);
+}
+
 // the SM-pair kernel works on 256 x 256 tiles, one per pair of SMs
 bool pair_fills_the_device(const cugl_context *ctx, const GemmOperands &op)
 {
@@ -114,6 +129,27 @@ bool gemmlowp_tcgen05_uses_pair(const cugl_context *ctx, const GemmOperands &op)
 {
     return gemmlowp_tcgen05_uses_pair_epi4(op) && !eight_epilogue_warps(op) && pair_fills_the_device(ctx, op) &&
            (op.block_n == 0 || op.block_n == 256);
+}
+
+// The batched launch runs the one-CTA row-major kernels.  What its products lose by that, one by one / in one launch, us:
+// * the SM-pair kernel, where K is long and one product's 256 x 256 tiles come in nearly whole waves of SM pairs:
+//   4 x 4096^3 199 / 207, 3 x 4096 x 2048 x 4096 86 / 90; not 4 x 3072^3 (99 / 96), nor 2 x 4096 x 4096 x 2048 (56.1 / 57.4, to
+//   float32 69.8 / 69.2), nor 2 x 2560 x 2560 x 2048 (1.4 waves: 33 / 27);
+// * the channel-major kernel for ragged 8-bit rows: 2 x 2099 x 3709 x 352 26.9 / 39.0, 3 x 4000 x 5001 x 256 80 / 119,
+//   2 x 1200 x 2001 x 400 18.4 / 21.4, 2 x 8000 x 1001 x 1000 46 / 51; not where one product's tiles are little more than
+//   a wave (4 x 1000 x 5001 x 256, 160 tiles: 50.1 / 46.7), nor a part of one above K = 512 (2 x 1200 x 3001 x 900: 29.7 / 27.8).
+// Everything else gains: 8 x 1024^3 50 / 13.3, 4 x 4096 x 4096 x 1024 103 / 65, 2 x 50176 x 256 x 64 24.8 / 18.8.
+bool gemmlowp_batch_by_product(const cugl_context *ctx, const GemmOperands &op, bool output_stage, bool allow_pair)
+{
+    auto whole_waves = [](long long tiles, long long slots) { return 5 * tiles >= 4 * slots * ((tiles + slots - 1) / slots); };
+    const long long sms = ctx->sm_count;
+    const long long pair_tiles = static_cast<long long>((op.M + 255) / 256) * ((op.N + 255) / 256);
+    if (allow_pair && op.K >= 4096 && gemmlowp_tcgen05_uses_pair(ctx, op) && whole_waves(pair_tiles, sms / 2))
+    {
+        return true;
+    }
+    const long long cm_tiles = static_cast<long long>((op.N + 127) / 128) * ((op.M + 255) / 256);
+    return output_stage && ragged_rows_channel_major(ctx, op) && (cm_tiles > sms ? whole_waves(cm_tiles, sms) : op.K <= 512);
 }
 
 cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,
@@ -141,7 +177,8 @@ cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, c
     {
         // Batches of attention-sized products: their tiles share one grid instead of each product filling its own
         // (16 products of 384 x 384 x 128: 6 - 18 tiles each).
-        return launch_gemmlowp_tcgen05_epi8(ctx, o, ep, false);
+        return batch_eight_epilogue_warps(o, ep.stage != CUGL_STAGE_NONE) ? launch_gemmlowp_tcgen05_epi8(ctx, o, ep, false)
+                                                                          : launch_gemmlowp_tcgen05_epi4(ctx, o, ep, false);
     }
     if (ep.stage == CUGL_STAGE_NONE && (ep.out_f32 != 0 || ep.accumulate != 0) && o.channel_major == 0)
     {

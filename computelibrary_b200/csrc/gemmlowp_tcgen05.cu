@@ -3867,15 +3867,16 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
     const bool s32 = ep.stage == CUGL_STAGE_NONE;
     if (op.batch > 1)
     {
-        // one launch over all products; only the eight-warp build holds these instantiations (gemmlowp_dispatch.cu)
-        if constexpr (kEpiWarps == 8)
+        // one launch over all products, with the rings of the single products below
+        if constexpr (kEpiWarps <= 8)
         {
+            constexpr bool kFour = kEpiWarps == 4;
             const int bn = op.block_n > 0 ? op.block_n : (op.N > 128 ? 256 : (op.N > 64 ? 128 : 64));
-            if (bn > 128) return s32 ? launch_variant<256, 3, 1, true, false, true>(ctx, op, ep) : launch_variant<256, 4, 1, false, false, true>(ctx, op, ep);
-            if (bn > 64) return s32 ? launch_variant<128, 5, 1, true, false, true>(ctx, op, ep) : launch_variant<128, 3, 2, false, false, true>(ctx, op, ep);
+            if (bn > 128) return s32 ? launch_variant<256, kFour ? 4 : 3, 1, true, false, true>(ctx, op, ep) : launch_variant<256, 4, 1, false, false, true>(ctx, op, ep);
+            if (bn > 64) return s32 ? launch_variant<128, kFour ? 3 : 5, kFour ? 2 : 1, true, false, true>(ctx, op, ep) : launch_variant<128, 3, 2, false, false, true>(ctx, op, ep);
             return s32 ? launch_variant<64, 3, 2, true, false, true>(ctx, op, ep) : launch_variant<64, 4, 2, false, false, true>(ctx, op, ep);
         }
-        return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "batched launches belong to the eight-warp build");
+        return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "batched launches belong to the four- and eight-warp builds");
     }
     if (op.split_k > 1)
     {

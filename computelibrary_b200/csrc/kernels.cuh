@@ -155,6 +155,8 @@ cugl_status launch_gemmlowp_simt(cugl_context *ctx, const GemmOperands &op, cons
 // TMA + tcgen05.mma.kind::i8 kernel.  Requires a, bt 16-byte aligned and lda, ldbt multiples of 16.
 bool        gemmlowp_tcgen05_supported(const GemmOperands &op);
 bool        gemmlowp_tcgen05_uses_pair(const cugl_context *ctx, const GemmOperands &op);
+// A batch whose products (op: one of them) are better off one by one: each takes a kernel that the batched launch lacks.
+bool        gemmlowp_batch_by_product(const cugl_context *ctx, const GemmOperands &op, bool output_stage, bool allow_pair);
 // allow_pair = false keeps to the one-CTA kernels (testing aid; all variants must agree bit for bit).
 cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,
                                     bool allow_pair = true);

@@ -230,11 +230,25 @@ struct GemmCore
         int64_t a_stride, d_stride;
         bool    shared_b;
     };
-    // One launch walks a whole batch through three-dimensional tensor maps (strides up to 2^40 bytes; the descriptor's
-    // validation keeps the products apart).  The generic kernel runs product by product.
-    bool one_launch(const Batch &bt) const
+    // One launch walks a batch through three-dimensional tensor maps (strides up to 2^40 bytes; the descriptor's validation
+    // keeps the products apart).  Product by product run the generic kernel, kernels that only exist for single products and
+    // were asked for by name, and products that are faster that way (gemmlowp_batch_by_product).
+    bool one_launch(const Batch &bt, int64_t lda, const void *d_dst, int64_t ldd) const
     {
-        return !force_simt && bt.a_stride < (1ll << 39) && bt.d_stride < (1ll << 39);
+        GemmOperands op{}; // one product, its A aligned as the copies are
+        op.a = op.bt = d_bt;
+        op.dst       = const_cast<void *>(d_dst);
+        op.lda       = round_up(lda, 16);
+        op.ldbt      = ldbt;
+        op.ldd       = ldd | bt.d_stride; // (only its alignment counts)
+        op.M = M, op.N = N, op.K = K;
+        op.epi_warps = epi_warps;
+        op.block_n   = block_n;
+        if (!uses_tcgen05(op) || bt.a_stride >= (1ll << 39) || bt.d_stride >= (1ll << 39) || epi_warps == 16 || channel_major != 0)
+        {
+            return false;
+        }
+        return b_off != 0 || !gemmlowp_batch_by_product(ctx, op, stage != CUGL_STAGE_NONE, allow_pair);
     }
 
     // rows x K product(s) against B copy b_copy (a batch with copies of its own: from b_copy on).
@@ -574,7 +588,7 @@ extern "C"
         const GemmCore::RawB  raw{d_b, d.ldb, d.b_batch_stride, plan->b_copies};
         const GemmCore::Batch all{d.batch, d.a_batch_stride, d.d_batch_stride, plan->b_copies == 1};
         const int32_t        *bias = d.has_bias ? d_bias : nullptr;
-        if (plan->collapse_batch || d.batch == 1 || plan->core.one_launch(all))
+        if (plan->collapse_batch || d.batch == 1 || plan->core.one_launch(all, d.lda, d_dst, d.ldd))
         {
             const bool one = plan->collapse_batch || d.batch == 1;
             CUGL_TRY(plan->core.gemm(d_a, d.lda, one ? d.M * d.batch : d.M, d_dst, d.ldd, bias, 0, 0, nullptr, 0, nullptr, 0, 255,
@@ -882,7 +896,8 @@ extern "C"
         const cugl_gemm_desc &d       = plan->desc;
         const GemmCore       &c = plan->core;
         const GemmCore::Batch all{d.batch, d.a_batch_stride, d.d_batch_stride, plan->b_copies == 1};
-        const bool one   = plan->collapse_batch || d.batch == 1 || c.one_launch(all);
+        const void *aligned = reinterpret_cast<const void *>(uintptr_t(256)); // (only known at run: assume an aligned destination)
+        const bool one   = plan->collapse_batch || d.batch == 1 || c.one_launch(all, d.lda, aligned, d.ldd);
         const bool rows  = c.b_off != 0 || (!c.force_simt && (d.lda & 15) != 0); // the operand preparation looks at A
         const bool new_b = !d.reshape_b_only_on_first_run;
         return one ? 1 + (rows || new_b ? 1 : 0) : d.batch * (rows ? 2 : 1) + (new_b ? 1 : 0);

@@ -162,6 +162,64 @@ def test_batch_in_one_launch(ctx, port, batch, M, N, K, ldd_pad):
         assert np.array_equal(acc, port.gemmlowp_core(a, b3, a_off, 0))
 
 
+def _batch_plan(ctx, batch, M, N, K, ldd_pad=0, **more):
+    desc, keep = capi.make_gemm_desc(M, N, K, capi.S8, capi.S8, capi.S8, 5, 0, batch=batch, ldd=N + ldd_pad, b_batch_stride=K * N,
+                                     multiplier=2 ** 30, shift=9, min_bound=-128, max_bound=127, **more)
+    return capi.GemmPlan(ctx, desc, keep)
+
+
+def _pair_shape(ctx):
+    return 256 * (ctx.sm_count // 4), 512  # a 256 x 256 tile for every pair of SMs (148 SMs: 74 tiles)
+
+
+def test_batch_routes(ctx):
+    """Which batches run in one launch: not those whose products fill the device with a kernel that the batched launch lacks
+    (the SM-pair kernel on long K, the channel-major one on ragged rows), and not those told to use such a kernel."""
+    M, N = _pair_shape(ctx)
+    rows = 256 * ctx.sm_count // 16  # with 1001 columns, eight 128-channel blocks: a channel-major tile for every second SM
+    many = 256 * (ctx.sm_count // 4)
+    for (m, n, k), launches in (((M, N, 4096), 3), ((M, N, 4080), 1), ((M - 512, N, 4096), 1), ((M + 2048, N, 4096), 1),
+                                ((rows + 256, 1001, 96), 3), ((rows + 256, 1008, 96), 1), ((rows - 256, 1001, 96), 1),
+                                ((rows + 256, 1001, 528), 1), ((many, 1001, 528), 3), ((many, 1001, 1040), 1), ((many // 2 + 256, 1001, 96), 1),
+                                ((384, 384, 128), 1), ((1024, 1024, 1024), 1)):
+        plan = _batch_plan(ctx, 3, m, n, k)
+        assert plan.launches == launches, (m, n, k)
+        plan.close()
+    for name, value, launches in (("set_epilogue_warps", 16, 3), ("set_epilogue_warps", 8, 1), ("set_epilogue_warps", 4, 1),
+                                  ("set_channel_major", 1, 3), ("set_tile_columns", 64, 1), ("force_simt", True, 3)):
+        plan = _batch_plan(ctx, 3, 300, 400, 256)
+        getattr(plan, name)(value)
+        assert plan.launches == launches, (name, value)
+        plan.close()
+    plan = _batch_plan(ctx, 3, M, N, 4096)
+    plan.allow_pair_kernel(False)
+    assert plan.launches == 1
+    plan.close()
+
+
+@pytest.mark.parametrize("batch,M,N,K,ldd_pad,kw", [
+    (2, 9472, 512, 4096, 0, {}), (2, 9216, 512, 4096, 0, {}), (2, 2500, 1001, 130, 0, {}), (2, 2100, 1001, 130, 3, {}), (2, 300, 520, 1279, 0, {}),
+    (3, 300, 520, 1280, 0, {}), (2, 260, 333, 4095, 0, {}), (2, 260, 333, 4096, 0, {}), (3, 129, 130, 1296, 16, {}), (5, 40, 60, 2000, 0, {}),
+    (3, 200, 300, 96, 0, dict(epi_warps=16)), (3, 200, 300, 96, 0, dict(epi_warps=4)), (3, 200, 304, 600, 0, dict(channel_major=1)),
+    (3, 200, 304, 1500, 0, dict(epi_warps=8)), (2, 5000, 2304, 64, 0, {})])
+def test_batches_on_both_sides_of_the_route_rules(ctx, port, batch, M, N, K, ldd_pad, kw):
+    """Products in one launch (four and eight epilogue warps, more than one wave of 256-column tiles) and one by one, against
+    the oracle on the first, the last and some rows in between; S32 and F32 too."""
+    rng = np.random.default_rng(batch * M + N + K)
+    a, b = q8_uniform(rng, (batch, M, K), np.int8), q8_uniform(rng, (batch, K, N), np.int8, -127, 127)
+    mult = rng.integers(2 ** 30, 2 ** 31 - 1, N).astype(np.int32)
+    shift = rng.integers(8, 14, N).astype(np.int32)
+    rows = np.unique(np.concatenate([np.arange(min(M, 40)), rng.integers(0, M, 20), np.arange(max(0, M - 40), M)]))
+    got, _ = gpu_gemmlowp(ctx, a, b, None, 5, 0, mult, shift, 3, -128, 127, np.int8, ldd_pad=ldd_pad, **kw)
+    raw, _ = gpu_gemmlowp(ctx, a, b, None, 5, 0, 0, 0, 0, 0, 0, np.int32, ldd_pad=4 * (ldd_pad // 4), **kw)
+    f, _ = gpu_gemmlowp(ctx, a, b, None, 5, 0, 0, 0, 0, 0, 0, np.float32, dequantize_scale=1.5e-3, b_constant=False, **kw)
+    for i in range(batch):
+        core = port.gemmlowp_core(a[i][rows], b[i], 5, 0)
+        assert np.array_equal(got[i][rows], port.gemmlowp_fused(a[i][rows], b[i], None, 5, 0, mult, shift, 3, -128, 127, np.int8)), i
+        assert np.array_equal(raw[i][rows], core), i
+        assert np.array_equal(f[i][rows], core.astype(np.float32) * np.float32(1.5e-3)), i
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (5, 63, 19), (129, 65, 130), (40, 4, 127), (33, 1000, 513), (200, 96, 3000)])
 def test_operand_preparation(ctx, port, M, N, K):
     """Row sums, realigned rows of A and the K-major copy of B with its column sums, over remainders of every tile edge;
