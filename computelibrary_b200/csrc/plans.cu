@@ -811,6 +811,12 @@ extern "C"
         op.M         = plan->collapse_batch ? plan->desc.M * plan->desc.batch : plan->desc.M;
         op.epi_warps = plan->core.epi_warps;
         op.block_n   = plan->core.block_n;
+        const cugl_gemm_desc &d = plan->desc;
+        if (d.batch > 1 && !plan->collapse_batch &&
+            plan->core.one_launch({d.batch, d.a_batch_stride, d.d_batch_stride, plan->b_copies == 1}, d.lda, op.a, d.ldd))
+        {
+            return "tcgen05"; // the batched launch has one CTA per tile
+        }
         return (plan->core.allow_pair && gemmlowp_tcgen05_uses_pair(plan->ctx, op)) ? "tcgen05_2cta" : "tcgen05";
     }
 

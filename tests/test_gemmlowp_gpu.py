@@ -197,6 +197,20 @@ def test_batch_routes(ctx):
     plan.close()
 
 
+def test_plan_kernel_of_a_batch(ctx):
+    """The kernel a batch's plan names is the one that runs: one CTA per tile in the batched launch, the SM pair only where
+    the products go one by one."""
+    M, N = _pair_shape(ctx)
+    for (m, n, k), kernel in (((M, N, 4096), "tcgen05_2cta"), ((M, N, 2048), "tcgen05"), ((2560, 2560, 1104), "tcgen05"), ((64, 64, 64), "tcgen05")):
+        plan = _batch_plan(ctx, 3, m, n, k)
+        assert plan.kernel == kernel, (m, n, k)
+        plan.close()
+    plan = _batch_plan(ctx, 3, M, N, 4096)
+    plan.allow_pair_kernel(False)
+    assert plan.kernel == "tcgen05"
+    plan.close()
+
+
 @pytest.mark.parametrize("batch,M,N,K,ldd_pad,kw", [
     (2, 9472, 512, 4096, 0, {}), (2, 9216, 512, 4096, 0, {}), (2, 2500, 1001, 130, 0, {}), (2, 2100, 1001, 130, 3, {}), (2, 300, 520, 1279, 0, {}),
     (3, 300, 520, 1280, 0, {}), (2, 260, 333, 4095, 0, {}), (2, 260, 333, 4096, 0, {}), (3, 129, 130, 1296, 16, {}), (5, 40, 60, 2000, 0, {}),
