@@ -904,7 +904,8 @@ extern "C"
         const GemmCore::Batch all{d.batch, d.a_batch_stride, d.d_batch_stride, plan->b_copies == 1};
         const void *aligned = reinterpret_cast<const void *>(uintptr_t(256)); // (only known at run: assume an aligned destination)
         const bool one   = plan->collapse_batch || d.batch == 1 || c.one_launch(all, d.lda, aligned, d.ldd);
-        const bool rows  = c.b_off != 0 || (!c.force_simt && (d.lda & 15) != 0); // the operand preparation looks at A
+        // the operand preparation looks at A: for its row sums, or because TMA cannot address it
+        const bool rows  = c.b_off != 0 || (!c.force_simt && ((d.lda | (d.batch > 1 && !plan->collapse_batch ? d.a_batch_stride : 0)) & 15) != 0);
         const bool new_b = !d.reshape_b_only_on_first_run;
         return one ? 1 + (rows || new_b ? 1 : 0) : d.batch * (rows ? 2 : 1) + (new_b ? 1 : 0);
     }

@@ -211,6 +211,14 @@ def test_plan_kernel_of_a_batch(ctx):
     plan.close()
 
 
+@pytest.mark.parametrize("gap,launches", [(0, 1), (16, 1), (5, 2), (8, 2)])
+def test_plan_launches_of_a_batch_with_a_gap(ctx, gap, launches):
+    """Products of A whose distance is not a multiple of 16 bytes are realigned first: a second launch."""
+    plan = _batch_plan(ctx, 3, 40, 64, 32, a_batch_stride=40 * 32 + gap)
+    assert plan.launches == launches
+    plan.close()
+
+
 @pytest.mark.parametrize("batch,M,N,K,ldd_pad,kw", [
     (2, 9472, 512, 4096, 0, {}), (2, 9216, 512, 4096, 0, {}), (2, 2500, 1001, 130, 0, {}), (2, 2100, 1001, 130, 3, {}), (2, 300, 520, 1279, 0, {}),
     (3, 300, 520, 1280, 0, {}), (2, 260, 333, 4095, 0, {}), (2, 260, 333, 4096, 0, {}), (3, 129, 130, 1296, 16, {}), (5, 40, 60, 2000, 0, {}),
