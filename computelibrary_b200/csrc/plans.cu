@@ -230,6 +230,16 @@ struct GemmCore
         int64_t a_stride, d_stride;
         bool    shared_b;
     };
+    // Products of a batch whose realigned copies of A share one launch: as many as kBatchCopyBytes hold, at least one.  (The
+    // copy of a single product was all the scratch a batch took when its products ran one by one; a launch over 32 MB of A is
+    // long enough not to miss the next product in it.)
+    static constexpr int64_t kBatchCopyBytes = 32ll << 20;
+    int copies_per_launch(int count) const
+    {
+        const int64_t fit = kBatchCopyBytes / (round_up(K, 16) * M);
+        return fit < 1 ? 1 : (fit < count ? static_cast<int>(fit) : count);
+    }
+
     // One launch walks a batch through three-dimensional tensor maps (strides up to 2^40 bytes; the descriptor's validation
     // keeps the products apart).  Product by product run the generic kernel, kernels that only exist for single products and
     // were asked for by name, and products that are faster that way (gemmlowp_batch_by_product).
@@ -523,7 +533,7 @@ extern "C"
         c.dst_dtype = desc->dst_dtype;
         apply_quant_fields(p, desc);
         c.lda_hint   = desc->lda;
-        c.tmp_a_rows = desc->M * desc->batch; // a batch is copied in one go
+        c.tmp_a_rows = desc->M * (p->collapse_batch ? desc->batch : c.copies_per_launch(desc->batch));
         cugl_status s = c.alloc(p->b_copies, desc->M * desc->batch);
         if (s == CUGL_SUCCESS)
         {
@@ -588,11 +598,24 @@ extern "C"
         const GemmCore::RawB  raw{d_b, d.ldb, d.b_batch_stride, plan->b_copies};
         const GemmCore::Batch all{d.batch, d.a_batch_stride, d.d_batch_stride, plan->b_copies == 1};
         const int32_t        *bias = d.has_bias ? d_bias : nullptr;
-        if (plan->collapse_batch || d.batch == 1 || plan->core.one_launch(all, d.lda, d_dst, d.ldd))
+        if (plan->collapse_batch || d.batch == 1)
         {
-            const bool one = plan->collapse_batch || d.batch == 1;
-            CUGL_TRY(plan->core.gemm(d_a, d.lda, one ? d.M * d.batch : d.M, d_dst, d.ldd, bias, 0, 0, nullptr, 0, nullptr, 0, 255,
-                                     new_b ? &raw : nullptr, one ? nullptr : &all));
+            CUGL_TRY(plan->core.gemm(d_a, d.lda, d.M * d.batch, d_dst, d.ldd, bias, 0, 0, nullptr, 0, nullptr, 0, 255, new_b ? &raw : nullptr));
+            plan->prepared = true;
+            return CUGL_SUCCESS;
+        }
+        if (plan->core.one_launch(all, d.lda, d_dst, d.ldd))
+        {
+            const bool unaligned = ((reinterpret_cast<uintptr_t>(d_a) | static_cast<uint64_t>(d.lda) | static_cast<uint64_t>(d.a_batch_stride)) & 15) != 0;
+            const int  group     = unaligned ? plan->core.copies_per_launch(d.batch) : d.batch;
+            for (int i = 0; i < d.batch; i += group)
+            {
+                GemmCore::Batch some = all;
+                some.count           = d.batch - i < group ? d.batch - i : group;
+                CUGL_TRY(plan->core.gemm(static_cast<const uint8_t *>(d_a) + i * d.a_batch_stride, d.lda, d.M,
+                                         static_cast<uint8_t *>(d_dst) + i * d.d_batch_stride, d.ldd, bias, plan->b_copies > 1 ? i : 0, i * d.M, nullptr,
+                                         0, nullptr, 0, 255, new_b && i == 0 ? &raw : nullptr, some.count > 1 ? &some : nullptr));
+            }
             plan->prepared = true;
             return CUGL_SUCCESS;
         }
@@ -907,7 +930,10 @@ extern "C"
         // the operand preparation looks at A: for its row sums, or because TMA cannot address it
         const bool rows  = c.b_off != 0 || (!c.force_simt && ((d.lda | (d.batch > 1 && !plan->collapse_batch ? d.a_batch_stride : 0)) & 15) != 0);
         const bool new_b = !d.reshape_b_only_on_first_run;
-        return one ? 1 + (rows || new_b ? 1 : 0) : d.batch * (rows ? 2 : 1) + (new_b ? 1 : 0);
+        if (!one) return d.batch * (rows ? 2 : 1) + (new_b ? 1 : 0);
+        const bool copied = !c.force_simt && d.batch > 1 && !plan->collapse_batch && ((d.lda | d.a_batch_stride) & 15) != 0;
+        const int  group  = copied ? c.copies_per_launch(d.batch) : d.batch;
+        return rows ? 2 * ((d.batch + group - 1) / group) : 1 + (new_b ? 1 : 0);
     }
 
     // ---- stand-alone kernels ---------------------------------------------------------------------

@@ -219,6 +219,26 @@ def test_plan_launches_of_a_batch_with_a_gap(ctx, gap, launches):
     plan.close()
 
 
+@pytest.mark.parametrize("batch,M,N,K,per_launch,own", [(5, 3000, 33, 5001, 2, True), (5, 3000, 33, 5001, 2, False), (3, 7000, 17, 4999, 1, True),
+                                                          (40, 50, 20, 33, 40, True)])
+def test_realigned_batches_take_bounded_scratch(ctx, port, batch, M, N, K, per_launch, own):
+    """The copies of A that a batch with unaligned rows needs at a time are bounded, whatever the batch: several launches where
+    they would be more than 32 MB, the last of them over fewer products; B that changes and B shared by all products."""
+    pitch = -(-K // 16) * 16
+    plan = _batch_plan(ctx, batch, M, N, K, a_batch_stride=M * K + 16)
+    assert plan.temp_bytes == -(-M * per_launch * pitch // 256) * 256 and plan.launches == 2 * -(-batch // per_launch)
+    plan.close()
+    rng = np.random.default_rng(batch * M + K)
+    a, b = q8_uniform(rng, (batch, M, K), np.uint8), q8_uniform(rng, (batch, K, N) if own else (K, N), np.uint8)
+    rows = np.unique(np.concatenate([np.arange(40), np.arange(M - 40, M)]))
+    for ldd_pad, const in ((0, not own), (3, True)):
+        got, _ = gpu_gemmlowp(ctx, a, b, None, -128, -120, 2 ** 30, 12, 3, 0, 255, np.uint8, ldd_pad=ldd_pad, b_constant=const, runs=2,
+                              temp_workspace=const)
+        for i in range(batch):
+            want = port.gemmlowp_fused(a[i][rows], b[i] if own else b, None, -128, -120, [2 ** 30], [12], 3, 0, 255, np.uint8)
+            assert np.array_equal(got[i][rows], want), (ldd_pad, const, i)
+
+
 @pytest.mark.parametrize("batch,M,N,K,ldd_pad,kw", [
     (2, 9472, 512, 4096, 0, {}), (2, 9216, 512, 4096, 0, {}), (2, 2500, 1001, 130, 0, {}), (2, 2100, 1001, 130, 3, {}), (2, 300, 520, 1279, 0, {}),
     (3, 300, 520, 1280, 0, {}), (2, 260, 333, 4095, 0, {}), (2, 260, 333, 4096, 0, {}), (3, 129, 130, 1296, 16, {}), (5, 40, 60, 2000, 0, {}),
