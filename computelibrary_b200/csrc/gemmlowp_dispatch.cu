@@ -182,7 +182,7 @@ cugl_status launch_gemmlowp_tcgen05(cugl_context *ctx, const GemmOperands &op, c
     }
     if (ep.stage == CUGL_STAGE_NONE && (ep.out_f32 != 0 || ep.accumulate != 0) && o.channel_major == 0)
     {
-        o.channel_major = -1; // read-modify-write of dst rows: the row-major epilogue does it with 128-bit accesses
+        o.channel_major = -1; // read-modify-write of dst rows: the row-major epilogue does it row by row, 128 bytes at a time
     }
     if (o.channel_major == 0)
     {

@@ -848,16 +848,66 @@ __device__ __noinline__ void flush_stage_words(const uint8_t *__restrict__ stage
     __syncwarp();
 }
 
-// 32-bit results, rows that are not 16-byte aligned: a staged chunk of 32 rows x 32 columns (128-byte swizzle) leaves as 32
-// consecutive words per row, one per lane.  o: this lane's column in row 0.
-__device__ __noinline__ void flush_raw_rows(const uint8_t *__restrict__ stage, uint8_t *__restrict__ o, int64_t ldd, int rows, int lane, EpilogueParams rp)
+// 32-bit results that no bulk tensor store takes (accumulation, several destinations, rows that are not 16-byte aligned): a
+// staged chunk of 32 rows x 32 columns (128-byte swizzle) leaves as 128 consecutive bytes per row.  d0: column 0 of row 0 of the
+// chunk; rows, cols: what of it exists; vec: its rows are 16-byte aligned.  Accumulation is bound by the latency of the old
+// values: those of every row of a step are on their way before the first store (one row after the other, whose load the
+// compiler may not lift over the store before it: 4096^3 441 us, 1024^3 23; now 83 and 8.8).
+__device__ __noinline__ void flush_raw_rows(const uint8_t *__restrict__ stage, uint8_t *__restrict__ d0, int64_t ldd, int rows, int cols, bool vec,
+                                            int lane, EpilogueParams rp)
 {
-#pragma unroll 4
-    for (int r = 0; r < rows; ++r)
+    if (vec && cols == 32) // eight lanes per row, four rows at a time
     {
-        const uint32_t w = *reinterpret_cast<const uint32_t *>(stage + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
-        uint32_t      *p = reinterpret_cast<uint32_t *>(o + r * ldd);
-        *p = raw_result_word(static_cast<int32_t>(w), rp.accumulate != 0 ? *p : 0u, rp);
+        const int piece = lane & 7, r0 = lane >> 3;
+        uint8_t  *d = d0 + r0 * ldd + 16 * piece;
+        uint4     old[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+        {
+            old[i] = make_uint4(0, 0, 0, 0);
+            if (rp.accumulate != 0 && r0 + 4 * i < rows) old[i] = *reinterpret_cast<const uint4 *>(d + 4 * i * ldd);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+        {
+            const int r = r0 + 4 * i;
+            if (r < rows)
+            {
+                const uint4 w = *reinterpret_cast<const uint4 *>(stage + r * 128 + ((piece ^ (r & 7)) << 4));
+                *reinterpret_cast<uint4 *>(d + 4 * i * ldd) =
+                    make_uint4(raw_result_word(static_cast<int32_t>(w.x), old[i].x, rp), raw_result_word(static_cast<int32_t>(w.y), old[i].y, rp),
+                               raw_result_word(static_cast<int32_t>(w.z), old[i].z, rp), raw_result_word(static_cast<int32_t>(w.w), old[i].w, rp));
+            }
+        }
+        return;
+    }
+    if (lane >= cols) return;
+    d0 += 4 * lane; // one word per lane
+    auto word = [&](int r) {
+        return static_cast<int32_t>(*reinterpret_cast<const uint32_t *>(stage + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3)));
+    };
+    if (rp.accumulate == 0)
+    {
+#pragma unroll 4
+        for (int r = 0; r < rows; ++r) *reinterpret_cast<uint32_t *>(d0 + r * ldd) = raw_result_word(word(r), 0u, rp);
+        return;
+    }
+    constexpr int kAhead = 16; // rows in flight
+#pragma unroll 1
+    for (int r0 = 0; r0 < rows; r0 += kAhead)
+    {
+        uint8_t *d = d0 + r0 * ldd;
+        uint32_t old[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+        {
+            old[i] = r0 + i < rows ? *reinterpret_cast<const uint32_t *>(d + i * ldd) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+        {
+            if (r0 + i < rows) *reinterpret_cast<uint32_t *>(d + i * ldd) = raw_result_word(word(r0 + i), old[i], rp);
+        }
     }
 }
 
@@ -992,11 +1042,11 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
     // 32-bit results: a chunk of 32 rows x 128 bytes leaves as one bulk tensor store as well.  A lane's own stores are
     // 16-byte pieces of one row each, a row pitch apart: eight times the load/store passes, and half a sector each.
     const bool    raw_tma = kS32Out && omap != nullptr; // warp-uniform (encode_raw_map: one destination, no accumulation)
-    // Anything else (accumulation, several destinations, rows that are not 16-byte aligned) goes through the stage too and
-    // leaves as 32 consecutive words per row, one per lane.
+    // Anything else (accumulation, several destinations, rows that are not 16-byte aligned) goes through the stage too
+    // (flush_raw_rows).
     const bool    raw_rows = kS32Out && kEpiWarps <= 8 && !raw_tma;
     auto raw_rows_flush = [&](const uint32_t *v, int c) {
-        const int n = n_first + c * 32 + lane;
+        const int n = n_first + c * 32;
         uint8_t  *row = stage + lane * 128;
         __syncwarp();
 #pragma unroll
@@ -1009,14 +1059,11 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
         rp.out_f32    = tp.raw_f32;
         rp.accumulate = tp.raw_accumulate;
         rp.dq_scale   = tp.raw_scale;
-        const int rows = min(32, tp.M - (m - lane));
-        if (n < tp.N)
+        const int     rows = min(32, tp.M - (m - lane)), cols = min(32, tp.N - n);
+        const int64_t off  = row_off - lane * tp.ldd + 4 * static_cast<int64_t>(n);
+        for (int x = -1; x < tp.n_extra; ++x)
         {
-            const int64_t off = row_off - lane * tp.ldd + 4 * static_cast<int64_t>(n);
-            for (int x = -1; x < tp.n_extra; ++x)
-            {
-                flush_raw_rows(stage, (x < 0 ? tp.dst : tp.extra_dst[x]) + off, tp.ldd, rows, lane, rp);
-            }
+            flush_raw_rows(stage, (x < 0 ? tp.dst : tp.extra_dst[x]) + off, tp.ldd, rows, cols, tp.vec_ok != 0, lane, rp);
         }
     };
     auto raw_stage_and_flush = [&](const uint32_t *v, int c) {

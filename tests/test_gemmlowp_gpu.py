@@ -654,6 +654,51 @@ def test_accumulate_and_dequantized_output(ctx, port, M, N, K, force_simt):
     assert np.array_equal(got, port.dequantize_s32(acc, scale, prev))
 
 
+@pytest.mark.parametrize("M,N,K", [(129, 33, 40), (257, 260, 600), (300, 1001, 1100), (95, 96, 2100), (1000, 31, 64), (31, 512, 1040)])
+@pytest.mark.parametrize("ldd_pad", [0, 3, 4])
+def test_accumulation_into_any_rows(ctx, port, M, N, K, ldd_pad):
+    """dst += result into rows of every alignment, with whole and partial chunks of 32 rows and 32 columns, one product and a
+    batch, four and eight epilogue warps and a cluster per tile (K = 2100)."""
+    rng = np.random.default_rng(M + N + K)
+    a, b = q8_uniform(rng, (2, M, K), np.int8), q8_uniform(rng, (2, K, N), np.int8)
+    cores = np.stack([port.gemmlowp_core(a[i], b[i], 7, -3) for i in range(2)])
+    init = rng.integers(-2 ** 20, 2 ** 20, (2, M, N)).astype(np.int32)
+    for n in (1, 2):
+        ops = (a[0], b[0]) if n == 1 else (a, b)
+        core, start = (cores[0], init[0]) if n == 1 else (cores, init)
+        got, _ = gpu_gemmlowp(ctx, *ops, None, 7, -3, 0, 0, 0, 0, 0, np.int32, ldd_pad=ldd_pad, accumulate=True, dst_init=start, runs=2)
+        assert np.array_equal(got, start + 2 * core), n
+        prev = start.astype(np.float32) * np.float32(0.25)
+        got, _ = gpu_gemmlowp(ctx, *ops, None, 7, -3, 0, 0, 0, 0, 0, np.float32, ldd_pad=ldd_pad, accumulate=True, dst_init=prev, dequantize_scale=0.125)
+        assert np.array_equal(got, prev + core.astype(np.float32) * np.float32(0.125)), n
+
+
+@pytest.mark.parametrize("M,N,K", [(4096, 4096, 4096), (2048, 2048, 1024), (2000, 2001, 1024)])
+def test_accumulation_is_no_chain_of_round_trips(ctx, M, N, K):
+    """Adding into dst reads its old values many rows at a time: it costs a small multiple of overwriting dst (1.2 - 1.8 measured),
+    not the 5 - 8 of a load that waits for the store of the row before it."""
+    import torch
+    a, b = (torch.randint(0, 256, (n,), dtype=torch.uint8, device="cuda") for n in (M * K, K * N))
+    dst = torch.zeros(M * N, dtype=torch.int32, device="cuda")
+    best = {}
+    for accumulate in (False, True):
+        desc, keep = capi.make_gemm_desc(M, N, K, capi.S8, capi.S8, capi.S32, 5, 0, capi.STAGE_NONE, accumulate=accumulate)
+        plan = capi.GemmPlan(ctx, desc, keep)
+        plan.prepare(b)
+        times = []
+        for _ in range(8):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(5):
+                plan.run(a, None, None, dst)
+            end.record()
+            end.synchronize()
+            times.append(start.elapsed_time(end))
+        best[accumulate] = min(times)
+        plan.close()
+    assert best[True] < 3 * best[False], best
+
+
 def test_validate_rules_of_the_raw_outputs():
     d, keep = capi.make_gemm_desc(8, 8, 8, capi.S8, capi.S8, capi.F32, stage=capi.STAGE_NONE)
     assert capi.gemm_validate(d)[0] == 6            # an F32 output needs a scale
