@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(kThreads) reduce_rows_kernel(const uint8_t *__
                                                                int K, int64_t lda, int32_t scalar,
                                                                int32_t *__restrict__ out)
 {
+    dependent_prologue(); // (launched by launch_prepare_operands)
     const int lane          = threadIdx.x & 31;
     const int warps_per_blk = kThreads / 32;
     for (int m = blockIdx.x * warps_per_blk + (threadIdx.x >> 5); m < M; m += gridDim.x * warps_per_blk)
@@ -849,6 +850,14 @@ cugl_status launch_prepare_operands(cugl_context *ctx, const OperandPrep &op)
         {
             p.row_lanes = kThreads;
             a_blocks    = static_cast<int>(all_rows);
+        }
+        else if (p.b_blocks == 0 && op.copy == nullptr && op.batch_a <= 1 && op.K > 512)
+        {
+            // Nothing but the sums of many long rows: the kernel that does only that holds more warps per SM (32768 x 1024:
+            // together with its product 15.4 us against 19.2, 10000 x 2064 13.7 / 16.1).
+            CUGL_CUDA_TRY(ctx, launch_dependent(ctx, reduce_rows_kernel, a_blocks, kThreads, 0, a_blocks, op.a, op.a_signed, op.rows, op.K, op.lda,
+                                                1, op.rowsum));
+            return check_cuda(ctx, cudaGetLastError(), "reduce_rows_kernel");
         }
     }
     if (p.b_blocks + a_blocks == 0) return CUGL_SUCCESS;

@@ -274,6 +274,24 @@ def test_operand_preparation(ctx, port, M, N, K):
             assert np.array_equal(acc, port.gemmlowp_core(a, b, 11, -7))
 
 
+@pytest.mark.parametrize("M,K", [(296, 513), (297, 513), (297, 512), (297, 528), (1500, 2064), (20000, 1040)])
+@pytest.mark.parametrize("lda_pad", [0, 16, 3])
+def test_row_sums_of_many_long_rows(ctx, port, M, K, lda_pad):
+    """Row sums alone (aligned rows), with the realigned copy, and a block per row, around the lines between them."""
+    import torch
+    rng = np.random.default_rng(M + K)
+    N, lda = 24, K + lda_pad
+    a, b = q8_uniform(rng, (M, lda), np.uint8), q8_uniform(rng, (K, N), np.uint8)
+    desc, keep = capi.make_gemm_desc(M, N, K, capi.U8, capi.U8, capi.S32, -128, -120, capi.STAGE_NONE, lda=lda)
+    plan = capi.GemmPlan(ctx, desc, keep)
+    plan.prepare(torch.from_numpy(b).cuda())
+    d_dst = torch.empty((M, N), dtype=torch.int32, device="cuda")
+    plan.run(torch.from_numpy(a).cuda(), None, None, d_dst)
+    ctx.sync()
+    plan.close()
+    assert np.array_equal(d_dst.cpu().numpy(), port.gemmlowp_core(np.ascontiguousarray(a[:, :K]), b, -128, -120))
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 2048), (33, 65, 2100), (49, 512, 4608), (97, 31, 16000), (130, 500, 1300), (300, 600, 2000),
                                    (256, 900, 2176), (128, 2112, 2048), (128, 2113, 2048), (128, 8, 2047)])
 def test_split_k(ctx, port, M, N, K):
