@@ -178,7 +178,7 @@ struct PrepParams
     OperandPrep op;
     int         b_strips, b_splits, b_blocks, k_per_split; // strips of 64 columns, K splits of k_per_split rows
     int         row_lanes; // lanes that share a row of A (kThreads: a block each)
-    bool        b_words, a_vec; // B rows 4-byte aligned / A rows 16-byte aligned
+    bool        a_vec; // A rows 16-byte aligned
 };
 
 // Four consecutive bytes starting at p, of which `valid` (>= 1) exist; the rest read as zero.
@@ -195,6 +195,7 @@ __device__ __forceinline__ uint32_t load_bytes4(const uint8_t *p, int valid)
 // rows of one 32-bit column word), transposes them with eight byte permutes and leaves four K-contiguous words in
 // shared memory; the tile goes out as 128 contiguous bytes per column.  The column sums come from the transposed words
 // (__dp4a); with one split per strip they are plain stores, else integer atomics on zeroed sums (exact in any order).
+template <bool kWords>
 __device__ __forceinline__ void prepare_b_strip(const PrepParams &p, int block, uint32_t (*tile)[33])
 {
     const OperandPrep &o     = p.op;
@@ -202,6 +203,7 @@ __device__ __forceinline__ void prepare_b_strip(const PrepParams &p, int block, 
     const int          strip = sz % p.b_strips, z = sz / p.b_strips;
     const int          n0 = strip * 64, k_begin = split * p.k_per_split, k_end = min(o.K, k_begin + p.k_per_split);
     const uint8_t     *b  = o.b + z * o.b_batch_stride;
+    const uint8_t     *b_end = b + static_cast<int64_t>(o.K - 1) * o.ldb + o.N;
     uint8_t           *bt = o.bt + static_cast<int64_t>(z) * o.N * o.ldbt;
     const int          w = threadIdx.x & 15, g = threadIdx.x >> 4; // column word, group of four rows (of 16)
     const int          n = n0 + 4 * w;
@@ -217,17 +219,39 @@ __device__ __forceinline__ void prepare_b_strip(const PrepParams &p, int block, 
             if (n < o.N)
             {
                 const uint8_t *src = b + static_cast<int64_t>(k) * o.ldb + n;
-                if (p.b_words && n + 4 <= o.N)
+                if (kWords && n + 4 <= o.N)
                 {
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         if (k + i < k_end) r[i] = __ldg(reinterpret_cast<const uint32_t *>(src + i * o.ldb));
                 }
-                else
+                else if (kWords)
                 {
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         if (k + i < k_end) r[i] = load_bytes4(src + i * o.ldb, o.N - n);
+                }
+                else
+                {
+                    // any alignment: two aligned words and a shift wherever both lie inside B (columns beyond N, whose bytes
+                    // belong to the next row, are neither stored nor summed), single bytes at its very ends
+                    uint32_t lo[4], hi[4];
+                    bool     inside[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                    {
+                        const uint8_t *q = src + i * o.ldb;
+                        q -= reinterpret_cast<uintptr_t>(q) & 3;
+                        inside[i] = k + i < k_end && q >= b && q + 8 <= b_end;
+                        lo[i] = inside[i] ? __ldg(reinterpret_cast<const uint32_t *>(q)) : 0u;
+                        hi[i] = inside[i] ? __ldg(reinterpret_cast<const uint32_t *>(q) + 1) : 0u;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                    {
+                        r[i] = __funnelshift_r(lo[i], hi[i], 8 * static_cast<int>(reinterpret_cast<uintptr_t>(src + i * o.ldb) & 3));
+                        if (!inside[i] && k + i < k_end) r[i] = load_bytes4(src + i * o.ldb, o.N - n);
+                    }
                 }
             }
             const uint32_t a0 = __byte_perm(r[0], r[1], 0x5140), a1 = __byte_perm(r[2], r[3], 0x5140);
@@ -393,6 +417,9 @@ __device__ __forceinline__ void prepare_a_rows(const PrepParams &p, int block, i
     }
 }
 
+// kWords: B's rows are 4-byte aligned (an instantiation of its own: the shifted loads cost the aligned ones registers and with them
+// blocks per SM, 4096 x 4096 10.3 -> 12.4 us)
+template <bool kWords>
 __global__ void __launch_bounds__(kThreads) prepare_operands_kernel(const __grid_constant__ PrepParams p)
 {
     __shared__ uint32_t tile[64][33];
@@ -400,7 +427,7 @@ __global__ void __launch_bounds__(kThreads) prepare_operands_kernel(const __grid
     const int block = static_cast<int>(blockIdx.x);
     if (block < p.b_blocks)
     {
-        prepare_b_strip(p, block, tile);
+        prepare_b_strip<kWords>(p, block, tile);
     }
     else if (p.row_lanes == kThreads)
     {
@@ -811,6 +838,7 @@ cugl_status launch_prepare_operands(cugl_context *ctx, const OperandPrep &op)
 {
     PrepParams p{};
     p.op = op;
+    bool b_words = true; // B rows 4-byte aligned
     if (op.b != nullptr && op.N > 0 && op.K > 0)
     {
         // One strip of 64 columns per block, all of K, when K is short or the strips alone give every SM six blocks: the column
@@ -829,7 +857,7 @@ cugl_status launch_prepare_operands(cugl_context *ctx, const OperandPrep &op)
         const int64_t blocks = strips * p.b_splits;
         if (blocks > INT32_MAX / 2) return fail(ctx, CUGL_UNSUPPORTED_CONFIG, "B operand: too many column strips");
         p.b_blocks = static_cast<int>(blocks);
-        p.b_words  = ((reinterpret_cast<uintptr_t>(op.b) | static_cast<uint64_t>(op.ldb) |
+        b_words    = ((reinterpret_cast<uintptr_t>(op.b) | static_cast<uint64_t>(op.ldb) |
                        static_cast<uint64_t>(op.batch_b > 1 ? op.b_batch_stride : 0)) & 3) == 0;
         if (p.b_splits > 1 && op.colsum != nullptr)
         {
@@ -861,7 +889,8 @@ cugl_status launch_prepare_operands(cugl_context *ctx, const OperandPrep &op)
         }
     }
     if (p.b_blocks + a_blocks == 0) return CUGL_SUCCESS;
-    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, prepare_operands_kernel, p.b_blocks + a_blocks, kThreads, 0, p.b_blocks + a_blocks, p));
+    CUGL_CUDA_TRY(ctx, launch_dependent(ctx, p.b_blocks == 0 || b_words ? prepare_operands_kernel<true> : prepare_operands_kernel<false>, p.b_blocks + a_blocks,
+                                        kThreads, 0, p.b_blocks + a_blocks, p));
     return check_cuda(ctx, cudaGetLastError(), "prepare_operands_kernel");
 }
 

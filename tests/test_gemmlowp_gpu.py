@@ -292,6 +292,26 @@ def test_row_sums_of_many_long_rows(ctx, port, M, K, lda_pad):
     assert np.array_equal(d_dst.cpu().numpy(), port.gemmlowp_core(np.ascontiguousarray(a[:, :K]), b, -128, -120))
 
 
+@pytest.mark.parametrize("K,N,ldb", [(1, 1, 1), (3, 2, 5), (130, 63, 63), (257, 65, 67), (513, 130, 131), (900, 429, 429), (131, 64, 66), (70, 7, 7)])
+@pytest.mark.parametrize("at", [0, 1, 2, 3])
+def test_preparing_b_of_any_alignment(ctx, port, K, N, ldb, at):
+    """B whose rows start anywhere: the first and last bytes of the matrix, which no aligned word inside it covers, included."""
+    import torch
+    rng = np.random.default_rng(K + N + at)
+    b, a = q8_uniform(rng, (K, ldb), np.int8), q8_uniform(rng, (5, K), np.int8)
+    size = (K - 1) * ldb + N
+    d_b = torch.full((size + 64,), 0x7F, dtype=torch.uint8, device="cuda")
+    d_b[at:at + size] = torch.from_numpy(b.view(np.uint8).reshape(-1)[:size]).cuda()
+    desc, keep = capi.make_gemm_desc(5, N, K, capi.S8, capi.S8, capi.S32, 7, -3, capi.STAGE_NONE, ldb=ldb)
+    plan = capi.GemmPlan(ctx, desc, keep)
+    plan.prepare(d_b[at:at + size])
+    d_dst = torch.empty((5, N), dtype=torch.int32, device="cuda")
+    plan.run(torch.from_numpy(a.view(np.uint8)).cuda(), None, None, d_dst)
+    ctx.sync()
+    plan.close()
+    assert np.array_equal(d_dst.cpu().numpy(), port.gemmlowp_core(a, np.ascontiguousarray(b[:, :N]), 7, -3))
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 2048), (33, 65, 2100), (49, 512, 4608), (97, 31, 16000), (130, 500, 1300), (300, 600, 2000),
                                    (256, 900, 2176), (128, 2112, 2048), (128, 2113, 2048), (128, 8, 2047)])
 def test_split_k(ctx, port, M, N, K):
