@@ -81,13 +81,15 @@ int pick_split(const cugl_context *ctx, const GemmOperands &op)
 // warps, whose lanes write eight neighbouring rows' bytes of their channel, is the fastest way out for them wherever its
 // 128-channel x 256-row tiles occupy half the device; against the row-major kernel's staged words (eight warps), us:
 // 2099 x 3709 x 352 13.5 / 20.7, 4000 x 5001 x 64 26.8 / 45.3, x 1000 39.7 / 54.7, 8000 x 301 x 256 8.4 / 11.8,
-// 500 x 6001 x 352 8.8 / 12.1.  Longer K belongs to the main loop and to the SM pair.
+// 500 x 6001 x 352 8.8 / 12.1, and with a single block of channels 100000 x 65 x 256 17.7 / 24.6, 20000 x 65 x 64 7.9 / 10.6; up
+// to 64 channels half of the tile and more is empty (100000 x 63 x 256 17.5 / 16.9, x 33 18.1 / 16.5, x 17 18.1 / 13.4).  The
+// bound on K is where the row-major kernels change, not a crossing: 2099 x 3709 x 2000 25 / 34.
 bool ragged_rows_channel_major(const cugl_context *ctx, const GemmOperands &op)
 {
     const bool      aligned = ((reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd)) & 15) == 0;
     const long long tiles   = static_cast<long long>((op.N + 127) / 128) * ((op.M + 255) / 256);
     return !aligned && op.channel_major == 0 && op.epi_warps == 0 && op.block_n == 0 && op.batch <= 1 && op.n_extra_dst == 0 &&
-           op.conv == nullptr && op.K <= kShortK && tiles >= ctx->sm_count / 2;
+           op.conv == nullptr && op.N > 64 && op.K <= kShortK && tiles >= ctx->sm_count / 2;
 }
 
 // Four or eight epilogue warps for a batch in one launch.  The batched kernels fill every wave, so that the shorter main

@@ -803,11 +803,34 @@ __device__ __noinline__ void flush_stage(const uint8_t *stage, uint8_t *d0, int6
 // shifted into place, with at most three single bytes at either end.  Per-lane byte stores wrote one byte of each of 32
 // rows per instruction, a sector each.
 // A call of its own: inlined, its addresses cost the drain of aligned rows registers.
-// d0: first valid byte of row 0 in global memory; rows, n: valid rows and bytes per row (<= 32 x kOutRowBytes).
+// Rows of at most kShortRow bytes that lie close together: a lane writes the row it has staged, byte by byte (a warp then fills whole
+// sectors; a wider pitch, as the last group of a wide row has, belongs to the words).  Spread over the lanes as words they took
+// longer than their bytes' way to memory: 100000 x 17 x 256 13.4 / 11.3 us, 20000 x 9 x 64 6.8 / 6.4 (x 31 still 6.8 / 6.7).
+// d0: first valid byte of row 0 in global memory; rows, n: valid rows and bytes per row (at most kOutRowBytes).
 // tma: the stage is in the tensor map's swizzle (dst would take bulk stores, it is the residual whose rows are not aligned).
 __device__ __noinline__ void flush_stage_words(const uint8_t *__restrict__ stage, uint8_t *__restrict__ d0, int64_t ldd, int rows, int n,
                                                int lane, bool tma)
 {
+    constexpr int kShortRow = 24, kShortPitch = 32;
+    if (n <= kShortRow && ldd <= kShortPitch) // warp-uniform
+    {
+        __syncwarp();
+        if (lane < rows)
+        {
+            const int      sw = stage_sw(lane, tma);
+            const uint4    w0 = *reinterpret_cast<const uint4 *>(stage + lane * kOutRowBytes + ((0 ^ sw) << 4));
+            const uint4    w1 = *reinterpret_cast<const uint4 *>(stage + lane * kOutRowBytes + ((1 ^ sw) << 4));
+            const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            uint8_t       *d = d0 + lane * ldd;
+#pragma unroll
+            for (int j = 0; j < kShortRow; ++j)
+            {
+                if (j < n) d[j] = static_cast<uint8_t>(w[j >> 2] >> (8 * (j & 3)));
+            }
+        }
+        __syncwarp();
+        return;
+    }
     constexpr int kAhead = 4; // steps in flight
     const int     shift = n <= 32 ? 3 : (n <= 64 ? 4 : 5); // lanes per row: 8, 16 or 32; the other lanes take further rows
     const int     i = lane & ((1 << shift) - 1), kRows = 32 >> shift;

@@ -375,6 +375,20 @@ def test_ragged_output_rows(ctx, port, M, N, K, ldd_pad):
         assert np.array_equal(got, port.gemmlowp_fused(a, b, bias, a_off, 0, mult, shift, 3, lo, hi, t)), t
 
 
+@pytest.mark.parametrize("M,N,ldd_pad", [(2600, 1, 0), (2600, 9, 0), (129, 17, 0), (2600, 24, 8), (2600, 24, 9), (131, 25, 0), (2600, 31, 1), (20000, 63, 0),
+                                         (20000, 64, 3), (19000, 65, 0), (300, 72, 0), (300, 152, 1)])
+@pytest.mark.parametrize("K", [40, 1300])
+def test_few_ragged_columns(ctx, port, M, N, ldd_pad, K):
+    """Rows of few unaligned bytes: written byte by byte where they lie close together, as words otherwise, the last short group
+    of a wider row, and the channel-major kernel from 65 columns on where there are enough rows."""
+    rng = np.random.default_rng(M + N + K)
+    a, b = q8_uniform(rng, (M, K), np.uint8), q8_uniform(rng, (K, N), np.int8, -127, 127)
+    mult, shift = rng.integers(2 ** 30, 2 ** 31 - 1, N).astype(np.int32), rng.integers(8, 14, N).astype(np.int32)
+    got, _ = gpu_gemmlowp(ctx, a, b, None, -128, 0, mult, shift, 3, 0, 255, np.uint8, ldd_pad=ldd_pad)
+    rows = np.unique(np.concatenate([np.arange(100), np.arange(M - 100, M), rng.integers(0, M, 300)]))
+    assert np.array_equal(got[rows], port.gemmlowp_fused(a[rows], b, None, -128, 0, mult, shift, 3, 0, 255, np.uint8))
+
+
 def test_run_twice_and_variable_b(ctx, port):
     """MultipleExecution (GEMMLowp.cpp:211-297): same plan, same output; B re-laid out per run when it is
     not constant (reshape_b_only_on_first_run = false)."""
