@@ -1221,7 +1221,13 @@ extern "C"
         const bool pointwise = desc->kw == 1 && desc->kh == 1 && desc->stride_x == 1 && desc->stride_y == 1 && desc->pad_left == 0 &&
                                desc->pad_right == 0 && desc->pad_top == 0 && desc->pad_bottom == 0;
         const bool countable = static_cast<int64_t>(desc->B) * desc->H * desc->W <= INT32_MAX; // pixels as 32-bit rows
-        p->pad_c = !p->fold && !pointwise && (desc->C % 16) != 0 && countable;
+        // Not where the padded patch no longer fits the implicit kernel's tap table (an explicit matrix is smaller without the
+        // padding: 2 x 64 x 64 x 1 -> 16, 33 x 33 39 us and 9 MB against 82 and 143), nor for the sixteenfold patch of a single channel
+        // under a larger window, measured with / without (s8 weights, us): 8 x 56 x 56 x 1 -> 200 5 x 5 28 / 16, 9 x 9 41 / 23;
+        // 4 x 64 x 64 x 1 -> 16 11 x 11 17.9 / 14.4; 3 x 3, 16 x 64 x 64 x 1 -> 64: 11.9 / 14.5.
+        const int64_t taps = static_cast<int64_t>(desc->kw) * desc->kh;
+        p->pad_c = !p->fold && !pointwise && (desc->C % 16) != 0 && countable && taps * round_up(desc->C, 16) <= kConvMaxK &&
+                   !(desc->C == 1 && taps >= 25);
         if (p->pad_c)
         {
             p->eC = static_cast<int>(round_up(desc->C, 16));

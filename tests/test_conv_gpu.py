@@ -457,6 +457,30 @@ def test_resident_weights_conv_vs_oracle(ctx, port, geom, batch):
         assert np.array_equal(got, want), (resident, np.argwhere(got != want)[:5])
 
 
+@pytest.mark.parametrize("H,C,k,kernel,matrix", [(64, 1, 33, "im2col", 1104), (12, 1, 3, "implicit", 0), (12, 1, 5, "im2col", 32), (12, 2, 5, "implicit", 0),
+                                                 (40, 3, 35, "im2col", 3680), (12, 1, 4, "implicit", 0)])
+@pytest.mark.parametrize("w_zp", [0, 120])
+def test_few_channels_under_large_windows(ctx, port, H, C, k, kernel, matrix, w_zp):
+    """Channels are padded to 16 only for the implicit kernel: where the padded patch is too long for it, or sixteen times the
+    patch of a single channel, the explicit matrix has the rows of the patch as it is."""
+    rng = np.random.default_rng(H * C + k)
+    src = q8_uniform(rng, (1, H, H, C), np.uint8)
+    wgt = q8_uniform(rng, (16, k, k, C), np.uint8 if w_zp else np.int8)
+    bias = rng.integers(-500, 501, 16).astype(np.int32)
+    mult, shift = f32_mults(port, 0.03, np.array([4e-3], np.float32), 0.03 * np.sqrt(k * k * C))
+    args = ((1, 1), (k // 2,) * 4, 128, w_zp, mult, shift, 5, 0, 255)
+    desc, keep = capi.make_conv_desc(1, H, H, C, 16, k, k, (1, 1), (k // 2,) * 4, (1, 1), capi.U8, capi.U8 if w_zp else capi.S8, 128, w_zp,
+                                     multiplier=int(mult[0]), shift=int(shift[0]), dst_zp=5, min_bound=0, max_bound=255, has_bias=True)
+    plan = capi.ConvPlan(ctx, desc, keep)
+    out = H + 2 * (k // 2) - k + 1
+    if kernel == "im2col":
+        sums = -(-4 * out * out // 256) * 256 if w_zp else 0
+        assert plan.temp_bytes == -(-out * out * matrix // 256) * 256 + sums
+    plan.close()
+    got = gpu_conv(ctx, src, wgt, bias, *args, want_kernel=kernel)
+    assert np.array_equal(got, port.conv2d_nhwc(src, wgt, bias, *args))
+
+
 @pytest.mark.parametrize("geom", [(16, 56, 56, 1, 64, 128), (13, 57, 59, 1, 40, 0), (11, 60, 61, 1, 64, 0), (50, 57, 59, 2, 64, 7)])
 def test_double_tile_conv_vs_oracle(ctx, port, geom):
     """3x3 x 64 convolutions large enough (more than 256 output pixels per SM) for the gather kernel's 256-pixel units,
