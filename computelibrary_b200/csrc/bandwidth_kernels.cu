@@ -171,7 +171,7 @@ __global__ void scale_vector_kernel(int32_t *v, int n, int32_t scalar)
 // behind them walk over the rows of A and produce row sums and, where the TMA engine cannot address A (base or pitch
 // not a multiple of 16 bytes), a copy with 16-byte rows.  The work is bound by launches when the operands are small
 // (16 products of 384 x 384 x 128 with a B that changes took 64 launches one after the other, 229 us; with this launch
-// and a batched product 10.3 us.  923 x 429 x 873 with unaligned rows: copy + reduction + product 24.6 us, now 20.1) and
+// and a batched product 10.5 us.  923 x 429 x 873 with unaligned rows: copy + reduction + product 24.6 us, now 14) and
 // by HBM when they are large.
 struct PrepParams
 {

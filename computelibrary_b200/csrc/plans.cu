@@ -1737,8 +1737,8 @@ extern "C"
         {
             return fail(plan->ctx, code, std::string("cugl_conv2d_update_quantization: ") + why);
         }
-        // the lowering was chosen for symmetric or asymmetric weights; a weights zero point appearing later would
-        // need the row sums the implicit kernel does not compute
+        // the lowering, its scratch and (implicit kernel) the instantiation with window sums were chosen for symmetric or for
+        // asymmetric weights
         if ((desc->w_zero_point != 0) != (o.w_zero_point != 0))
         {
             return fail(plan->ctx, CUGL_UNSUPPORTED_CONFIG,

@@ -111,8 +111,9 @@ CUGL_API cugl_status cugl_context_withhold_copy_once(cugl_context *ctx, int k_bl
 /* The tensor-core kernels are launched with programmatic stream serialization (on by default): a kernel lets the next
  * one in the stream start its prologue (barrier set-up, tensor-memory allocation) while its own last tiles finish, and
  * every kernel waits for its predecessor's completion (griddepcontrol.wait) before its first access to global memory.
- * A stream that is being captured into a CUDA graph gets plain launches (measured faster there).  0 restores plain
- * stream order everywhere.  No
+ * The operand preparation and the short kernels between the products (at most one block per SM) are launched the same way.
+ * A stream that is being captured into a CUDA graph gets programmatic edges for short launches only (at most four tiles or
+ * blocks per SM; measured slower for longer ones).  0 restores plain stream order everywhere.  No
  * reference counterpart (the NE scheduler runs its kernels back to back on the host threads). */
 CUGL_API cugl_status cugl_context_set_dependent_launch(cugl_context *ctx, int on);
 
