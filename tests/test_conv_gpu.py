@@ -358,6 +358,42 @@ def test_conv_update_quantization_and_bound_workspace(ctx, port):
         plan.close()
 
 
+@pytest.mark.parametrize("C,k,s", [(17, 3, 2), (21, 1, 1), (48, 3, 1), (5, 3, 1), (40, 1, 2)])
+@pytest.mark.parametrize("implicit", [True, False])
+def test_workspace_of_asymmetric_and_padded_convolutions(ctx, port, C, k, s, implicit):
+    """The shares of a bound workspace (pixel or row sums, padded or realigned input, im2col matrix) under asymmetric weights:
+    nothing outside it is written, and the padding and the out-of-image sums follow the zero points when these change."""
+    import torch
+    rng = np.random.default_rng(C * 10 + k)
+    B, H, W, OFM, pad = 2, 9, 11, 24, k // 2
+    src, wgt = q8_uniform(rng, (B, H, W, C), np.uint8), q8_uniform(rng, (OFM, k, k, C), np.uint8)
+    bias = rng.integers(-3000, 3001, OFM).astype(np.int32)
+    mult, shift = f32_mults(port, 0.03, np.array([5e-3], np.float32), 0.03 * np.sqrt(k * k * C))
+    d_src, d_w, d_b = torch.from_numpy(src).cuda(), torch.from_numpy(wgt).cuda(), torch.from_numpy(bias).cuda()
+
+    def desc_for(izp, wzp):
+        return capi.make_conv_desc(B, H, W, C, OFM, k, k, (s, s), (pad,) * 4, (1, 1), capi.U8, capi.U8, izp, wzp, multiplier=int(mult[0]),
+                                   shift=int(shift[0]), dst_zp=7, min_bound=0, max_bound=255, has_bias=True)
+    desc, keep = desc_for(128, 120)
+    plan = capi.ConvPlan(ctx, desc, keep)
+    plan.allow_implicit(implicit)
+    guard, n = 512, plan.temp_bytes
+    assert n > 0
+    ws = torch.full((guard + n + guard,), 0x77, dtype=torch.uint8, device="cuda")
+    plan.bind_temp(ws[guard:], n)
+    plan.prepare(d_w)
+    wo, ho = plan.out_dims()
+    d_dst = torch.empty((B, ho, wo, OFM), dtype=torch.uint8, device="cuda")
+    for izp, wzp in ((128, 120), (90, 3), (0, 255)):
+        if (izp, wzp) != (128, 120):
+            plan.update_quantization(*desc_for(izp, wzp))
+        plan.run(d_src, d_b, d_dst)
+        ctx.sync()
+        assert np.array_equal(d_dst.cpu().numpy(), port.conv2d_nhwc(src, wgt, bias, (s, s), (pad,) * 4, izp, wzp, mult, shift, 7, 0, 255)), (izp, wzp)
+    assert (ws[:guard] == 0x77).all() and (ws[guard + n:] == 0x77).all()
+    plan.close()
+
+
 def test_transpose_batched_is_the_nchw_nhwc_permute(ctx):
     import torch
     rng = np.random.default_rng(6)

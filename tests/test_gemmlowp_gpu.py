@@ -389,6 +389,54 @@ def test_few_ragged_columns(ctx, port, M, N, ldd_pad, K):
     assert np.array_equal(got[rows], port.gemmlowp_fused(a[rows], b, None, -128, 0, mult, shift, 3, 0, 255, np.uint8))
 
 
+@pytest.mark.parametrize("batch,M,N,K", [(1, 100, 200, 300), (1, 64, 70, 2100), (1, 500, 257, 1000), (3, 40, 96, 640), (16, 384, 384, 128)])
+def test_captured_products_with_changing_b(port, batch, M, N, K):
+    """A product and a batch whose B (and A) change, recorded into a CUDA graph: operand preparation (with zeroed column sums in
+    front of it where K is split over blocks), product and a second product that reads the first one's result, replayed with
+    new operands."""
+    import torch
+    import computelibrary_b200 as cl
+    rng = np.random.default_rng(batch * M + N + K)
+    stream = torch.cuda.Stream()
+    ctx = cl.Context(0, stream.cuda_stream)
+    mult, shift = capi.calculate_quantized_multiplier(np.float32(0.5 / (73 * np.sqrt(K))))
+    mult2, shift2 = capi.calculate_quantized_multiplier(np.float32(0.5 / (73 * np.sqrt(N))))
+
+    def plan_for(m, n, k, mu, sh):
+        desc, keep = capi.make_gemm_desc(m, n, k, capi.U8, capi.U8, capi.U8, -128, -120, batch=batch, b_batch_stride=k * n if batch > 1 else 0,
+                                         multiplier=mu, shift=sh, offset=100, min_bound=0, max_bound=255, b_constant=False)
+        return capi.GemmPlan(ctx, desc, keep)
+    first, second = plan_for(M, N, K, mult, shift), plan_for(M, 48, N, mult2, shift2)
+    shapes = ((batch, M, K), (batch, K, N), (batch, N, 48))
+    with torch.cuda.stream(stream):
+        d_a, d_b, d_c = (torch.empty(s, dtype=torch.uint8, device="cuda") for s in shapes)
+        d_mid, d_out = (torch.empty((batch, M, n), dtype=torch.uint8, device="cuda") for n in (N, 48))
+
+        def step():
+            first.run(d_a, d_b, None, d_mid)
+            second.run(d_mid, d_c, None, d_out)
+        step()
+    ctx.sync()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        step()
+    for _ in range(3):
+        a, b, c = (q8_uniform(rng, s, np.uint8) for s in shapes)
+        with torch.cuda.stream(stream):
+            for d, h in ((d_a, a), (d_b, b), (d_c, c)):
+                d.copy_(torch.from_numpy(h))
+            graph.replay()
+        ctx.sync()
+        for i in range(batch):
+            mid = port.gemmlowp_fused(a[i], b[i], None, -128, -120, [mult], [shift], 100, 0, 255, np.uint8)
+            assert np.array_equal(d_mid[i].cpu().numpy(), mid), i
+            assert np.array_equal(d_out[i].cpu().numpy(), port.gemmlowp_fused(mid, c[i], None, -128, -120, [mult2], [shift2], 100, 0, 255, np.uint8)), i
+    del graph
+    first.close()
+    second.close()
+    ctx.close()
+
+
 def test_run_twice_and_variable_b(ctx, port):
     """MultipleExecution (GEMMLowp.cpp:211-297): same plan, same output; B re-laid out per run when it is
     not constant (reshape_b_only_on_first_run = false)."""
