@@ -799,6 +799,40 @@ __device__ __noinline__ void flush_stage(const uint8_t *stage, uint8_t *d0, int6
     __syncwarp();
 }
 
+// The same to several destinations: every piece is read from the stage once and stored to all of them (one destination after the
+// other, 1024 x 512 x 512 to eight: 9.2 against 7.2 us).  off: first valid byte of row 0 in every destination.
+__device__ __forceinline__ void flush_stage_many(const uint8_t *stage, const TileParams &tp, int64_t off, int rows, int n, int lane)
+{
+    __syncwarp();
+    const int p = lane & (kOutPieces - 1);
+#pragma unroll 2
+    for (int it = 0; it < kOutPieces; ++it)
+    {
+        const int r = it * (32 / kOutPieces) + lane / kOutPieces;
+        if (r < rows && p * 16 < n)
+        {
+            const uint4   val = *reinterpret_cast<const uint4 *>(stage + r * kOutRowBytes + ((p ^ stage_sw(r, false)) << 4));
+            const int64_t o   = off + r * tp.ldd + p * 16;
+            if (p * 16 + 16 <= n)
+            {
+                *reinterpret_cast<uint4 *>(tp.dst + o) = val;
+                for (int x = 0; x < tp.n_extra; ++x) *reinterpret_cast<uint4 *>(tp.extra_dst[x] + o) = val;
+            }
+            else
+            {
+                const uint32_t w[4] = {val.x, val.y, val.z, val.w};
+                for (int j = 0; j < n - p * 16; ++j)
+                {
+                    const uint8_t b = static_cast<uint8_t>(w[j >> 2] >> (8 * (j & 3)));
+                    tp.dst[o + j]   = b;
+                    for (int x = 0; x < tp.n_extra; ++x) tp.extra_dst[x][o + j] = b;
+                }
+            }
+        }
+    }
+    __syncwarp();
+}
+
 // The same for rows that are not 16-byte aligned (N or the pitch odd): a row of the stage leaves as aligned 32-bit words,
 // shifted into place, with at most three single bytes at either end.  Per-lane byte stores wrote one byte of each of 32
 // rows per instruction, a sector each.
@@ -1047,7 +1081,11 @@ __device__ __forceinline__ void release_accumulators(const AccRelease &r, int la
 // Shared epilogue of both kernels: one warp drains NCOLS consecutive columns (a multiple of 32) of its
 // 32 accumulator rows from tensor memory, applies the offset / bias terms and the output stage, and
 // stores.  The tensor-memory load of chunk i+1 is issued before chunk i is processed.
-template <int NCOLS, bool kS32Out, int kMode>
+// kTo: kToMany for several destinations (the push all-gather), whose pieces are stored to all of them by inlined code.  The drain of
+// a single destination keeps its loop over them all the same: the compiler allocates the kernels' registers better with it than
+// without (2 x 4096 x 4096 x 1024 35.7 against 40.4 us, 32 x 112 x 112 x 3 -> 64 3x3 35.5 / 37.7).
+constexpr int kToOne = 0, kToMany = 1;
+template <int NCOLS, bool kS32Out, int kMode, int kTo = kToOne>
 __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s_col, const TileParams &tp,
                                                   const EpilogueParams &ep, int m, int n_first, int32_t row_term,
                                                   uint8_t *stage, int lane, const AccRelease &rel,
@@ -1145,7 +1183,12 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
                 if (rows > 0 && cols > 0)
                 {
                     const int64_t off = row_off - lane * tp.ldd + n_group;
-                    for (int x = -1; x < tp.n_extra; ++x)
+                    if (kTo == kToMany && tp.vec_ok != 0)
+                    {
+                        flush_stage_many(stage, tp, off, rows, cols, lane);
+                        return;
+                    }
+                    for (int x = -1; x < tp.n_extra; ++x) // (several only with kToMany; see there)
                     {
                         uint8_t *d0 = (x < 0 ? tp.dst : tp.extra_dst[x]) + off;
                         if (tp.vec_ok != 0) flush_stage(stage, d0, tp.ldd, rows, cols, lane, tma);
@@ -1882,7 +1925,7 @@ __device__ __forceinline__ void epilogue_warp_tile_cm(uint32_t tmem_acc, const T
 // kGroups = 2: the eight epilogue warps form two groups of four that drain alternate tiles, each warp all columns
 // of its 32 rows (narrow tiles, whose time is latency rather than work).
 // kGivenRowTerm: the caller has worked out the row term itself (window sums of a convolution)
-template <int BLOCK_N, bool kS32Out, int kGroups = 1, bool kGivenRowTerm = false>
+template <int BLOCK_N, bool kS32Out, int kGroups = 1, bool kGivenRowTerm = false, int kTo = kToOne>
 __device__ __forceinline__ void epilogue_warp_tile(uint32_t tmem_acc, const int4 *s_col, const TileParams &tp,
                                                    const EpilogueParams &ep, int warp, int lane, int m0, int n0,
                                                    uint8_t *out_stage, const AccRelease &rel,
@@ -1899,27 +1942,27 @@ __device__ __forceinline__ void epilogue_warp_tile(uint32_t tmem_acc, const int4
     const uint32_t t_addr  = tmem_acc + (static_cast<uint32_t>(quad * 32) << 16) + half * NCOLS;
     if (tp.mode == kStagePack && !kS32Out)
     {
-        drain_accumulator<NCOLS, kS32Out, kStagePack>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
+        drain_accumulator<NCOLS, kS32Out, kStagePack, kTo>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
                                                       stage, lane, rel, omap, z);
     }
     else if (tp.mode == kStagePackS && !kS32Out)
     {
-        drain_accumulator<NCOLS, kS32Out, kStagePackS>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
+        drain_accumulator<NCOLS, kS32Out, kStagePackS, kTo>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
                                                        stage, lane, rel, omap, z);
     }
     else if (tp.mode == kStageWide && !kS32Out)
     {
-        drain_accumulator<NCOLS, kS32Out, kStageWide>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
+        drain_accumulator<NCOLS, kS32Out, kStageWide, kTo>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
                                                       stage, lane, rel, omap, z);
     }
     else if (tp.mode == kStageGeneric)
     {
-        drain_accumulator<NCOLS, kS32Out, kStageGeneric>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS,
+        drain_accumulator<NCOLS, kS32Out, kStageGeneric, kTo>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS,
                                                          row_term, stage, lane, rel, omap, z);
     }
     else
     {
-        drain_accumulator<NCOLS, kS32Out, kStageFast>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
+        drain_accumulator<NCOLS, kS32Out, kStageFast, kTo>(t_addr, s_col + half * NCOLS, tp, ep, m, n0 + half * NCOLS, row_term,
                                                       stage, lane, rel, omap, z);
     }
 }
@@ -2040,7 +2083,8 @@ struct SmemPlan
 // three-dimensional tensor maps, whose bounds keep a ragged last row block inside its own product.
 // kSplit: the tp.split CTAs of a cluster work on one tile, each on its own range of K (epilogue_warp_tile_split); one
 // tile per cluster.
-template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kCM, int ACC, bool kPairTma = false, bool kBatched = false, bool kSplit = false>
+template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kCM, int ACC, bool kPairTma = false, bool kBatched = false, bool kSplit = false,
+          int kTo = kToOne>
 __global__ void __launch_bounds__(kThreads, 1)
     gemmlowp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                             const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_res,
@@ -2417,7 +2461,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         constexpr int  kStride  = 1;
         // Two buffers only: with 128-column tiles in four buffers, pairs (0, 1) and (2, 3) drained by sixteen warps while
         // the MMA warp fills the other pair, the same layers measured slower (802816 x 256 x 64: 164 against 133 us).
-        constexpr bool kCanPair = !kCM && !kS32Out && kGroups == 1 && ACC == 2 && !kBatched && !kSplit;
+        constexpr bool kCanPair = kTo == kToOne && !kCM && !kS32Out && kGroups == 1 && ACC == 2 && !kBatched && !kSplit;
         int            skip     = -1; // ordinal of a tile already drained as the partner of an earlier one
         uint32_t       n_res_pairs = 0; // kPairTma: pairs whose residual this warp has fetched (phase of its barrier)
         for (int tile = first_tile(); tile < num_tiles; tile += tile_step(), ++ti)
@@ -2534,7 +2578,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                     else
                     {
-                        epilogue_warp_tile<BLOCK_N, kS32Out, kGroups>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane, m0, n0,
+                        epilogue_warp_tile<BLOCK_N, kS32Out, kGroups, false, kTo>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane, m0, n0,
                                                                       smem + P::OFF_OUT, rel, omap);
                     }
                 }
@@ -2611,7 +2655,7 @@ struct SmemPlan2
     static constexpr int TMEM_COLS = 2 * BLOCK_N;
 };
 
-template <int STAGES, int KSUB, bool kS32Out>
+template <int STAGES, int KSUB, bool kS32Out, int kTo = kToOne>
 __global__ void __launch_bounds__(kThreads, 1)
     gemmlowp_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                  const __grid_constant__ CUtensorMap tmap_b,
@@ -2918,12 +2962,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const AccRelease rel{map_to_cta(tempty_bar(as), 0), 0u, true}; // one arrival per warp, at the leader
                 if (half < 0)
                 {
-                    epilogue_warp_tile<BLOCK_N, kS32Out>(tmem_base + as * BLOCK_N, s_col, tp, ep, warp, lane, m0, n0,
+                    epilogue_warp_tile<BLOCK_N, kS32Out, 1, false, kTo>(tmem_base + as * BLOCK_N, s_col, tp, ep, warp, lane, m0, n0,
                                                          smem + P::OFF_OUT, rel, tp.tma_store != 0 ? &tmap_out : nullptr);
                 }
                 else
                 {
-                    epilogue_warp_tile<BLOCK_N / 2, kS32Out>(tmem_base + as * BLOCK_N, s_col, tp, ep, warp, lane, m0, n0,
+                    epilogue_warp_tile<BLOCK_N / 2, kS32Out, 1, false, kTo>(tmem_base + as * BLOCK_N, s_col, tp, ep, warp, lane, m0, n0,
                                                              smem + P::OFF_OUT, rel, tp.tma_store != 0 ? &tmap_out : nullptr);
                 }
                 __syncwarp();
@@ -3629,8 +3673,8 @@ bool conv_tma_supported(const GemmOperands &op)
            (cv.kw - 1) * cv.dil_x < 256 && (cv.kh - 1) * cv.dil_y < 256 && get_encode_im2col_fn() != nullptr;
 }
 
-template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kPairTma = false, bool kBatched = false, bool kSplit = false>
-cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
+template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kPairTma, bool kBatched, bool kSplit, int kTo>
+cugl_status launch_variant_to(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
 {
     constexpr int ACC = BLOCK_N <= 128 ? 4 : 2; // narrow tiles: four accumulator buffers in the 512 columns
     using P = SmemPlan<BLOCK_N, STAGES, KSUB, ACC, kPairTma, 0, kS32Out && kEpiWarps <= 8>;
@@ -3667,7 +3711,7 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
             return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the residual tiles");
         }
     }
-    auto kernel = gemmlowp_tcgen05_kernel<BLOCK_N, STAGES, KSUB, kS32Out, false, ACC, kPairTma, kBatched, kSplit>;
+    auto kernel = gemmlowp_tcgen05_kernel<BLOCK_N, STAGES, KSUB, kS32Out, false, ACC, kPairTma, kBatched, kSplit, kTo>;
     static bool attr_set[64] = {}; // per instantiation and device
     if (!attr_set[ctx->device & 63])
     {
@@ -3718,6 +3762,16 @@ cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const Epil
     return check_cuda(ctx, cudaGetLastError(), "gemmlowp_tcgen05_kernel");
 }
 
+template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out, bool kPairTma = false, bool kBatched = false, bool kSplit = false>
+cugl_status launch_variant(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
+{
+    if constexpr (!kPairTma && !kBatched && !kSplit) // (those have one destination)
+    {
+        if (op.n_extra_dst > 0) return launch_variant_to<BLOCK_N, STAGES, KSUB, kS32Out, false, false, false, kToMany>(ctx, op, ep);
+    }
+    return launch_variant_to<BLOCK_N, STAGES, KSUB, kS32Out, kPairTma, kBatched, kSplit, kToOne>(ctx, op, ep);
+}
+
 // Channel-major launch: weights on the 128-row side of the tile, BLOCK_N rows of the activation matrix on the other.
 template <int BLOCK_N, int STAGES, int KSUB, bool kS32Out>
 cugl_status launch_variant_cm(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
@@ -3765,7 +3819,7 @@ cugl_status launch_variant_cm(cugl_context *ctx, const GemmOperands &op, const E
 }
 
 #if CUGL_TC_PAIR_BUILD
-template <int STAGES, int KSUB, bool kS32Out>
+template <int STAGES, int KSUB, bool kS32Out, int kTo>
 cugl_status launch_variant_2cta(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep)
 {
     using P = SmemPlan2<STAGES, KSUB>;
@@ -3788,7 +3842,7 @@ cugl_status launch_variant_2cta(cugl_context *ctx, const GemmOperands &op, const
     {
         return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the output tiles");
     }
-    auto kernel = gemmlowp_tcgen05_2cta_kernel<STAGES, KSUB, kS32Out>;
+    auto kernel = gemmlowp_tcgen05_2cta_kernel<STAGES, KSUB, kS32Out, kTo>;
     static bool attr_set[64] = {}; // per instantiation and device
     if (!attr_set[ctx->device & 63])
     {
@@ -3968,7 +4022,8 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
 #if CUGL_TC_PAIR_BUILD
     if (allow_pair && CUGL_TC_NAME(gemmlowp_tcgen05_uses_pair)(op) && !(op.conv != nullptr && op.conv->C == 64)) // (64-byte-swizzle tiles: one-CTA kernels)
     {
-        return s32 ? launch_variant_2cta<3, 2, true>(ctx, op, ep) : launch_variant_2cta<3, 2, false>(ctx, op, ep);
+        if (op.n_extra_dst > 0) return s32 ? launch_variant_2cta<3, 2, true, kToMany>(ctx, op, ep) : launch_variant_2cta<3, 2, false, kToMany>(ctx, op, ep);
+        return s32 ? launch_variant_2cta<3, 2, true, kToOne>(ctx, op, ep) : launch_variant_2cta<3, 2, false, kToOne>(ctx, op, ep);
     }
 #else
     (void)allow_pair;
@@ -3991,7 +4046,7 @@ cugl_status CUGL_TC_NAME(launch_gemmlowp_tcgen05)(cugl_context *ctx, const GemmO
 #if CUGL_TC_FULL_BUILD
     // K of at most one 128-byte block: a tile is a single stage, so one-block stages and a ring twice as deep keep
     // twice as many tiles' operands in flight (the loads of such layers are bound by latency, not by bandwidth)
-    const bool one_block = op.K <= BLOCK_K && !s32;
+    const bool one_block = op.K <= BLOCK_K && !s32 && op.n_extra_dst == 0;
     if (block_n > 64)
     {
         if (one_block) return launch_variant<128, 6, 1, false>(ctx, op, ep);

@@ -605,6 +605,38 @@ def test_epilogue_builds_and_stage_encodings(ctx, port, shape, epi_warps):
     assert np.array_equal(got, port.gemmlowp_fused(a, bu, bias, -7, -9, [1099511552], [8], 10, 0, 255, np.uint8))
 
 
+@pytest.mark.parametrize("M,N,K,pad,n", [(300, 520, 96, 8, 3), (300, 520, 96, 0, 8), (2400, 1024, 64, 0, 2), (129, 333, 200, 0, 4), (257, 96, 1300, 0, 8),
+                                         (4736, 512, 1040, 16, 3), (70, 17, 640, 0, 5)])
+@pytest.mark.parametrize("epi_warps", [0, 4, 8, 16])
+def test_run_multi_every_store_path(ctx, port, M, N, K, pad, n, epi_warps):
+    """The push to several destinations on every kernel that writes them: whole and ragged pieces, unaligned and short rows, wide
+    and narrow tiles, the SM pair; canary bytes between and behind the rows of each destination; 32-bit results as well."""
+    import torch
+    rng = np.random.default_rng(M + N + K + n)
+    a, b = q8_uniform(rng, (M, K), np.int8), q8_uniform(rng, (K, N), np.int8, -127, 127)
+    mult, shift = rng.integers(2 ** 30, 2 ** 31 - 1, N).astype(np.int32), rng.integers(8, 14, N).astype(np.int32)
+    rows = np.unique(np.concatenate([np.arange(min(M, 70)), np.arange(max(0, M - 70), M)]))
+    d_a, d_b = torch.from_numpy(a.view(np.uint8)).cuda(), torch.from_numpy(b.view(np.uint8)).cuda()
+    for out, want in ((capi.S8, port.gemmlowp_fused(a[rows], b, None, 5, 0, mult, shift, 3, -128, 127, np.int8)),
+                      (capi.S32, port.gemmlowp_core(a[rows], b, 5, 0))):
+        size = want.dtype.itemsize
+        ldd = N * size + 4 * pad
+        stage = dict(stage=capi.STAGE_NONE) if out == capi.S32 else dict(multipliers=mult, shifts=shift, offset=3, min_bound=-128, max_bound=127)
+        desc, keep = capi.make_gemm_desc(M, N, K, capi.S8, capi.S8, out, 5, 0, ldd=ldd, **stage)
+        plan = capi.GemmPlan(ctx, desc, keep)
+        plan.set_epilogue_warps(epi_warps)
+        plan.prepare(d_b)
+        dsts = [torch.full((M * ldd + 64,), 0xA5, dtype=torch.uint8, device="cuda") for _ in range(n)]
+        plan.run_multi(d_a, None, dsts)
+        ctx.sync()
+        for d in dsts:
+            got = d.cpu().numpy()
+            body = got[:M * ldd].reshape(M, ldd)
+            assert np.array_equal(np.ascontiguousarray(body[rows][:, :N * size]).view(want.dtype), want), out
+            assert (body[:, N * size:] == 0xA5).all() and (got[M * ldd:] == 0xA5).all(), out
+        plan.close()
+
+
 def test_run_multi_destinations_eight_epilogue_warps(ctx, port):
     """The staged multi-destination store of the eight-warp build (64-byte row segments), ragged N and M."""
     import torch
