@@ -1084,7 +1084,7 @@ __device__ __forceinline__ void release_accumulators(const AccRelease &r, int la
 // kTo: kToMany for several destinations (the push all-gather), whose pieces are stored to all of them by inlined code.  The drain of
 // a single destination keeps its loop over them all the same: the compiler allocates the kernels' registers better with it than
 // without (2 x 4096 x 4096 x 1024 35.7 against 40.4 us, 32 x 112 x 112 x 3 -> 64 3x3 35.5 / 37.7).
-constexpr int kToOne = 0, kToMany = 1;
+constexpr int kToOne = 0, kToMany = 1, kToBulk = 2; // (bulk: one, and every group by a bulk tensor store: whole groups, N a multiple of 16)
 template <int NCOLS, bool kS32Out, int kMode, int kTo = kToOne>
 __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s_col, const TileParams &tp,
                                                   const EpilogueParams &ep, int m, int n_first, int32_t row_term,
@@ -1096,7 +1096,8 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
     const int64_t row_off = dst_off + static_cast<int64_t>(m) * tp.ldd;
     uint8_t      *drow    = tp.dst + row_off;
     // omap: the warp's 32 rows x kOutRowBytes leave as one bulk tensor store from its staging area (one destination)
-    const bool    tma     = !kS32Out && omap != nullptr && tp.n_extra == 0; // warp-uniform
+    const bool    tma     = kTo == kToBulk || (!kS32Out && omap != nullptr && tp.n_extra == 0); // warp-uniform
+    static_assert(kTo != kToBulk || (!kS32Out && NCOLS % kOutRowBytes == 0), "bulk stores take whole groups");
     // builds of up to eight warps: everything leaves through the stage
     const bool    staged  = !kS32Out && (kEpiWarps <= 8 || tp.n_extra > 0 || tma); // warp-uniform
     // chunk c of the warp's columns into the stage; the group goes out when it is complete
@@ -1173,7 +1174,7 @@ __device__ __forceinline__ void drain_accumulator(uint32_t t_addr, const int4 *s
             // ragged end of a 200-byte row wrote bytes 200..207 too), so a group that crosses N leaves through the
             // lanes unless N itself ends on such a unit.
             const int n_group = n_first + first * 32;
-            if (tma && ncols == kOutRowBytes && (n_group + kOutRowBytes <= tp.N || (tp.N & 15) == 0))
+            if (kTo == kToBulk || (tma && ncols == kOutRowBytes && (n_group + kOutRowBytes <= tp.N || (tp.N & 15) == 0)))
             {
                 flush_stage_tma(stage, omap, m - lane, n_first + first * 32, lane, z);
             }
@@ -3076,7 +3077,11 @@ constexpr int kConvThreads  = kThreads + 32 * kGatherWarps;
 // pixels, two 128-row tiles that share every hand-over -- one stage barrier, one commit and one accumulator-ready signal
 // for both, where a 64-column tile is bound by exactly those (the tensor pipe is busy a quarter of the time).  A stage
 // holds the patches of both tiles for one K step; epilogue group g drains tile g of every unit.
-template <int BLOCK_N, int STAGES, int KSUB, int ACC, int RESB = 0, int MT = 1>
+// kAsym: weights with a zero point, i.e. a window sum per output pixel (window_sum).  An instantiation of its own: as a run-time
+// test the call took registers from symmetric weights too (10 x 40 x 40 x 32 -> 96, 5x5 8.4 -> 8.55 us, now 8.26; 41 x 26 x 26 x 16 -> 208, 3x3 / 2 6.84 -> 7.03, 6.69).
+// kTo = kToBulk where every staged group leaves as a bulk tensor store: the drain then holds no call (wide tiles only; 32 x 56 x 56 x
+// 64 -> 256 1x1 / 2: 10.2 -> 9.9 us, narrow ones gain nothing).
+template <int BLOCK_N, int STAGES, int KSUB, int ACC, int RESB = 0, int MT = 1, bool kAsym = false, int kTo = kToOne>
 __global__ void __launch_bounds__(kConvThreads, 1)
     gemmlowp_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_out,
                                  const __grid_constant__ TileParams tp, const EpilogueParams ep,
@@ -3344,16 +3349,21 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 if (kGroups == 1) epi_barrier();
                 else epi_group_barrier(group);
             }
-            const int      m_row    = m0 + (warp & 3) * 32 + lane;
-            const int32_t  row_term = (ep.rowsum != nullptr && m_row < tp.M) ? ep.b_off * window_sum(ep.rowsum, m_row, cg) : 0;
+            int32_t row_term = 0;
+            if constexpr (kAsym)
+            {
+                const int m_row = m0 + (warp & 3) * 32 + lane;
+                row_term        = m_row < tp.M ? ep.b_off * window_sum(ep.rowsum, m_row, cg) : 0;
+            }
             ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(as_first), aph, s_abort, DEV_TIMEOUT_EPILOGUE, tp.spin_limit));
             if (ok)
             {
                 tc_fence_after();
                 if (et == 0) trace_event(tp.trace, ti, 4);
                 const AccRelease rel{tempty_bar(as), 0u, false};
-                epilogue_warp_tile<BLOCK_N, false, kGroups, true>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane, m0, n0,
-                                                                  smem + P::OFF_OUT, rel, tp.tma_store != 0 ? &tmap_out : nullptr,
+                epilogue_warp_tile<BLOCK_N, false, kGroups, true, kTo>(tmem_base + as * BLOCK_N, g_col, tp, ep, warp, lane, m0, n0,
+                                                                       smem + P::OFF_OUT, rel,
+                                                                       kTo == kToBulk || tp.tma_store != 0 ? &tmap_out : nullptr,
                                                                   -1, row_term);
                 if (et == 0) trace_event(tp.trace, ti, 5);
                 __syncwarp();
@@ -3882,8 +3892,8 @@ cugl_status launch_variant_2cta(cugl_context *ctx, const GemmOperands &op, const
 #endif // CUGL_TC_PAIR_BUILD
 
 #if CUGL_TC_FULL_BUILD
-template <int BLOCK_N, int STAGES, int KSUB, int ACC, int RESB = 0, int MT = 1>
-cugl_status launch_conv_variant(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,
+template <int BLOCK_N, int STAGES, int KSUB, int ACC, int RESB, int MT, bool kAsym, int kTo>
+cugl_status launch_conv_kernel(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,
                                 const ConvOperands &cv)
 {
     using P = SmemPlan<BLOCK_N, STAGES, MT * KSUB, ACC, false, RESB>;
@@ -3903,7 +3913,7 @@ cugl_status launch_conv_variant(cugl_context *ctx, const GemmOperands &op, const
     {
         return fail(ctx, CUGL_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed for the output tiles");
     }
-    auto        kernel = gemmlowp_conv_tcgen05_kernel<BLOCK_N, STAGES, KSUB, ACC, RESB, MT>;
+    auto        kernel = gemmlowp_conv_tcgen05_kernel<BLOCK_N, STAGES, KSUB, ACC, RESB, MT, kAsym, kTo>;
     static bool attr_set[64] = {};
     if (!attr_set[ctx->device & 63])
     {
@@ -3955,6 +3965,24 @@ cugl_status launch_conv_variant(cugl_context *ctx, const GemmOperands &op, const
     tp.tma_store = tma_store ? 1 : 0;
     CUGL_CUDA_TRY(ctx, launch_dependent(ctx, kernel, grid, kConvThreads, kDynBytes, tiles, map_b, map_out, tp, ep, cg));
     return check_cuda(ctx, cudaGetLastError(), "gemmlowp_conv_tcgen05_kernel");
+}
+
+template <int BLOCK_N, int STAGES, int KSUB, int ACC, int RESB = 0, int MT = 1>
+cugl_status launch_conv_variant(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep, const ConvOperands &cv)
+{
+    if (ep.rowsum != nullptr)
+    {
+        return launch_conv_kernel<BLOCK_N, STAGES, KSUB, ACC, RESB, MT, true, kToOne>(ctx, op, ep, cv);
+    }
+    if constexpr (BLOCK_N > 64) // (their warps' columns are whole groups)
+    {
+        // what encode_out_map asks for
+        if (op.tma_store >= 0 && op.n_extra_dst == 0 && ((reinterpret_cast<uintptr_t>(op.dst) | static_cast<uint64_t>(op.ldd | op.N)) & 15) == 0)
+        {
+            return launch_conv_kernel<BLOCK_N, STAGES, KSUB, ACC, RESB, MT, false, kToBulk>(ctx, op, ep, cv);
+        }
+    }
+    return launch_conv_kernel<BLOCK_N, STAGES, KSUB, ACC, RESB, MT, false, kToOne>(ctx, op, ep, cv);
 }
 #endif // CUGL_TC_FULL_BUILD
 } // namespace

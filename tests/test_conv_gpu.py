@@ -517,6 +517,24 @@ def test_few_channels_under_large_windows(ctx, port, H, C, k, kernel, matrix, w_
     assert np.array_equal(got, port.conv2d_nhwc(src, wgt, bias, *args))
 
 
+@pytest.mark.parametrize("B,H,C,OFM,k,s", [(16, 56, 64, 64, 3, 1), (13, 57, 64, 40, 3, 1), (7, 30, 64, 64, 3, 1), (3, 21, 48, 24, 3, 2), (2, 33, 64, 130, 3, 1),
+                                           (3, 25, 32, 256, 3, 1), (2, 20, 128, 200, 3, 1), (4, 28, 96, 320, 1, 2)])
+@pytest.mark.parametrize("w_zp", [120, 0])
+def test_gather_kernels_with_and_without_window_sums(ctx, port, B, H, C, OFM, k, s, w_zp):
+    """Every instantiation of the gather kernel -- resident weights, units of two tiles (16 x 56 x 56 and 13 x 57 x 57), reloading ones of
+    64, 128 and 256 columns, whole and ragged output rows -- with the window sums of asymmetric weights and without."""
+    rng = np.random.default_rng(B * H + C + OFM)
+    src = q8_uniform(rng, (B, H, H, C), np.uint8)
+    wgt = q8_uniform(rng, (OFM, k, k, C), np.uint8 if w_zp else np.int8)
+    bias = rng.integers(-5000, 5001, OFM).astype(np.int32)
+    mult, shift = f32_mults(port, 0.03, np.exp(rng.uniform(np.log(1e-3), np.log(1e-2), 1 if w_zp else OFM)).astype(np.float32), 0.03 * np.sqrt(k * k * C))
+    args = ((s, s), (k // 2,) * 4, 128, w_zp, mult, shift, 3, 0, 255)
+    want = port.conv2d_nhwc(src, wgt, bias, *args)
+    for kw in ({}, dict(resident_weights=False), dict(double_tile=False)):
+        got = gpu_conv(ctx, src, wgt, bias, *args, want_kernel="implicit", tma_im2col=False, **kw)
+        assert np.array_equal(got, want), kw
+
+
 @pytest.mark.parametrize("geom", [(16, 56, 56, 1, 64, 128), (13, 57, 59, 1, 40, 0), (11, 60, 61, 1, 64, 0), (50, 57, 59, 2, 64, 7)])
 def test_double_tile_conv_vs_oracle(ctx, port, geom):
     """3x3 x 64 convolutions large enough (more than 256 output pixels per SM) for the gather kernel's 256-pixel units,
