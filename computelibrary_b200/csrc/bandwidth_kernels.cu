@@ -620,6 +620,38 @@ __global__ void __launch_bounds__(kThreads) spread_channels_kernel(const uint8_t
     }
 }
 
+// ---- sums over the windows of a convolution ----------------------------------------------------
+// From the channel sums of the input pixels to the patch sum of every output pixel; eight lanes share a window, four loads in
+// flight each.  Bound by launch and load latency (1 x 14 x 14, 11 x 11 with 16 channels: 16.2 us for all three launches, 32.8 with the sums inside the product).
+__global__ void __launch_bounds__(kThreads) window_sums_kernel(const int32_t *__restrict__ pixel_sums, int32_t *__restrict__ out, int M,
+                                                               const __grid_constant__ ConvOperands cv, FastDiv div_wo, FastDiv div_ho, FastDiv div_kw)
+{
+    dependent_prologue();
+    const int sub = threadIdx.x & 7, taps = cv.kw * cv.kh;
+    for (int64_t m0 = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x - (threadIdx.x & 31)) >> 3; m0 < M;
+         m0 += static_cast<int64_t>(gridDim.x) * (kThreads / 8)) // the warp's four pixels
+    {
+        const int m  = min(static_cast<int>(m0) + static_cast<int>((threadIdx.x & 31) >> 3), M - 1);
+        const int q  = fast_div(m, div_wo), xo = m - q * cv.Wo;
+        const int bi = fast_div(q, div_ho), yo = q - bi * cv.Ho;
+        const int y0 = yo * cv.sy - cv.pad_t, x0 = xo * cv.sx - cv.pad_l;
+        const int32_t *image = pixel_sums + static_cast<int64_t>(bi) * cv.H * cv.W;
+        int32_t        sum   = 0;
+#pragma unroll 4
+        for (int t = sub; t < taps; t += 8)
+        {
+            const int ky = fast_div(t, div_kw), kx = t - ky * cv.kw;
+            const int y = y0 + ky * cv.dil_y, x = x0 + kx * cv.dil_x;
+            const bool in = static_cast<unsigned>(y) < static_cast<unsigned>(cv.H) && static_cast<unsigned>(x) < static_cast<unsigned>(cv.W);
+            sum += in ? __ldg(image + static_cast<int64_t>(y) * cv.W + x) : cv.pad_sum;
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        if (sub == 0) out[m] = sum; // (lanes beyond the last pixel repeat it: the same value twice)
+    }
+}
+
 template <int VEC>
 __global__ void __launch_bounds__(kThreads) im2col_nhwc_kernel(const uint8_t *__restrict__ src,
                                                                uint8_t *__restrict__ dst, int C, int W, int H,
@@ -966,6 +998,15 @@ cugl_status launch_spread_channels(cugl_context *ctx, const void *d_src, void *d
     spread_channels_kernel<<<blocks, kThreads, 0, ctx->stream>>>(static_cast<const uint8_t *>(d_src), static_cast<uint8_t *>(d_dst), rows,
                                                                  taps, C, Cp, ldd);
     return check_cuda(ctx, cudaGetLastError(), "spread_channels_kernel");
+}
+
+cugl_status launch_window_sums(cugl_context *ctx, const int32_t *d_pixel_sums, const ConvOperands &cv, int M, int32_t *d_out)
+{
+    if (M <= 0) return CUGL_SUCCESS;
+    const int blocks = grid_for(static_cast<int64_t>(M) * 8, ctx->sm_count);
+    CUGL_CUDA_TRY(ctx, launch_blocks(ctx, window_sums_kernel, blocks, d_pixel_sums, d_out, M, cv, make_fastdiv(cv.Wo), make_fastdiv(cv.Ho),
+                                     make_fastdiv(cv.kw)));
+    return check_cuda(ctx, cudaGetLastError(), "window_sums_kernel");
 }
 
 cugl_status launch_im2col_nhwc(cugl_context *ctx, const void *d_src, void *d_dst, int C, int W, int H, int B, int kw,

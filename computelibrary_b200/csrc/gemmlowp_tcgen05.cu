@@ -3023,6 +3023,7 @@ struct ConvGeom
     int            C, W, H, kw, kh, sx, sy, pad_l, pad_t, dil_x, dil_y, Wo, Ho;
     FastDiv        div_wo, div_ho;
     int32_t        pad_sum; // channel sum of an out-of-image tap (asymmetric weights)
+    bool           row_sums; // EpilogueParams::rowsum: per output pixel instead of per input pixel
 };
 
 // Asymmetric weights: sum over the patch of output pixel m, from the channel sums of the input pixels.  A kh x kw window
@@ -3353,7 +3354,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             if constexpr (kAsym)
             {
                 const int m_row = m0 + (warp & 3) * 32 + lane;
-                row_term        = m_row < tp.M ? ep.b_off * window_sum(ep.rowsum, m_row, cg) : 0;
+                row_term        = m_row < tp.M ? ep.b_off * (cg.row_sums ? __ldg(ep.rowsum + m_row) : window_sum(ep.rowsum, m_row, cg)) : 0;
             }
             ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(as_first), aph, s_abort, DEV_TIMEOUT_EPILOGUE, tp.spin_limit));
             if (ok)
@@ -3959,7 +3960,8 @@ cugl_status launch_conv_kernel(cugl_context *ctx, const GemmOperands &op, const 
     cg.Ho    = cv.Ho;
     cg.div_wo = make_fastdiv(cv.Wo);
     cg.div_ho = make_fastdiv(cv.Ho);
-    cg.pad_sum = cv.pad_sum;
+    cg.pad_sum  = cv.pad_sum;
+    cg.row_sums = cv.row_sums;
     const int tiles = ((op.M + MT * BLOCK_M - 1) / (MT * BLOCK_M)) * ((op.N + BLOCK_N - 1) / BLOCK_N); // units of MT tiles
     const int grid  = tiles < ctx->sm_count ? tiles : ctx->sm_count;
     tp.tma_store = tma_store ? 1 : 0;

@@ -123,8 +123,17 @@ struct ConvOperands
     // asymmetric weights: EpilogueParams::rowsum holds the channel sum of every input PIXEL, the kernel adds up the window
     // of each output pixel; pad_sum is the channel sum of an out-of-image tap
     int32_t        pad_sum;
+    // row_sums: EpilogueParams::rowsum holds the sum of every output pixel's patch already (launch_window_sums)
+    bool           row_sums;
     int            C, W, H, B, kw, kh, sx, sy, pad_l, pad_t, dil_x, dil_y, Wo, Ho;
 };
+// Filter taps up to which the implicit kernel adds up the windows of pixel sums itself (window_sum: nine loads at a time, per
+// tile, behind the main loop's back); above, a launch of its own spreads them over the device, where the main loop is too short
+// to hide them (few channels, and up to 64 with few tiles).  Inside / apart, us: 1 x 14 x 14 x 16 -> 32 5 x 5 12.2 / 14, 7 x 7 17.1 / 12.2,
+// 11 x 11 32.8 / 16.2; 1 x 14 x 14 x 64 -> 32 7 x 7 17.6 / 18, 11 x 11 33.4 / 27.2; 8 x 28 x 28 x 128 -> 200 7 x 7 27.1 / 32.8.
+constexpr int kWindowTaps = 25;
+// out[m] = sum over the kh x kw window of output pixel m of the pixel sums, out-of-image taps counting cv.pad_sum
+cugl_status launch_window_sums(cugl_context *ctx, const int32_t *d_pixel_sums, const ConvOperands &cv, int M, int32_t *d_out);
 bool        gemmlowp_conv_tcgen05_supported(const GemmOperands &op, const ConvOperands &cv);
 // op.a / op.lda are unused: the A tile comes from cv.src.  M = B*Ho*Wo, K = kh*kw*C.
 cugl_status launch_gemmlowp_conv_tcgen05(cugl_context *ctx, const GemmOperands &op, const EpilogueParams &ep,

@@ -1108,6 +1108,18 @@ struct cugl_conv_plan
     {
         return static_cast<int64_t>(desc.B) * eH * eW;
     }
+    // asymmetric weights with a large window (kWindowTaps): the row-sum vector holds the pixel sums and, from sums_offset() on,
+    // the patch sums
+    int64_t sums_offset() const
+    {
+        return round_up(pixels(), 4);
+    }
+    bool windows_apart() const
+    {
+        const int taps = ekw * ekh;
+        return implicit && desc.w_zero_point != 0 && sums_offset() + M <= INT32_MAX &&
+               ((eC <= 32 && taps > kWindowTaps) || (eC <= 64 && taps > 2 * kWindowTaps && M <= 4096));
+    }
     // fused residual addition (cugl_conv2d_plan_set_residual): clamp bounds of the saturating form
     bool residual_set = false;
     int  res_floor = 0, res_cap = 255;
@@ -1262,7 +1274,7 @@ extern "C"
         p->implicit = !p->skip_im2col && (p->eC % 16) == 0 && p->K <= kConvMaxK &&
                       static_cast<int64_t>(p->eH) * p->eW * p->eC < (1ll << 31) && (desc->w_zero_point == 0 || countable);
         // row sums: one per output pixel, or (implicit kernel) one channel sum per input pixel
-        const int64_t n_sums = p->implicit && countable && p->pixels() > p->M ? p->pixels() : p->M;
+        const int64_t n_sums = p->windows_apart() ? p->sums_offset() + p->M : (p->implicit && countable && p->pixels() > p->M ? p->pixels() : p->M);
         cugl_status   s      = c.alloc(1, static_cast<int>(n_sums));
         if (s == CUGL_SUCCESS)
         {
@@ -1491,6 +1503,7 @@ extern "C"
             cv.dil_y  = d.dil_y;
             cv.Wo     = plan->Wo;
             cv.Ho     = plan->Ho;
+            cv.row_sums = false;
             const int zp_byte = d.src_zero_point & 0xff;
             cv.pad_sum        = plan->eC * (c.a_signed ? static_cast<int8_t>(zp_byte) : zp_byte);
             // Input zero point 0 and whole 128-channel blocks: the TMA unit builds the patch tiles itself (im2col-mode
@@ -1509,6 +1522,13 @@ extern "C"
             }
             if (gemmlowp_conv_tcgen05_supported(op, cv))
             {
+                if (pixel_sums != nullptr && plan->windows_apart())
+                {
+                    int32_t *patch_sums = pixel_sums + plan->sums_offset();
+                    CUGL_TRY(launch_window_sums(plan->ctx, pixel_sums, cv, op.M, patch_sums));
+                    pixel_sums  = patch_sums;
+                    cv.row_sums = true;
+                }
                 return launch_gemmlowp_conv_tcgen05(plan->ctx, op, c.epilogue(d.has_bias ? d_bias : nullptr, 0, pixel_sums), cv);
             }
         }
@@ -1709,7 +1729,7 @@ extern "C"
         const int fold = plan->fold ? 1 : 0;
         if (plan->implicit && plan->allow_implicit)
         {
-            return fold + (plan->pad_c || plan->core.b_off != 0 ? 1 : 0) + 1;
+            return fold + (plan->pad_c || plan->core.b_off != 0 ? 1 : 0) + (plan->windows_apart() ? 1 : 0) + 1;
         }
         const bool rows = plan->core.b_off != 0 || (plan->skip_im2col && (plan->desc.C & 15) != 0);
         return fold + (plan->pad_c ? 1 : 0) + (plan->skip_im2col ? 0 : 1) + 1 + (rows ? 1 : 0);

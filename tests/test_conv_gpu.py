@@ -535,6 +535,49 @@ def test_gather_kernels_with_and_without_window_sums(ctx, port, B, H, C, OFM, k,
         assert np.array_equal(got, want), kw
 
 
+@pytest.mark.parametrize("H,C,k,s,pad,dil", [(14, 16, 5, 1, 2, 1), (14, 16, 7, 1, 3, 1), (15, 32, 9, 2, 4, 1), (20, 64, 7, 1, 3, 1), (20, 64, 8, 1, 2, 1), (13, 17, 6, 1, 0, 2),
+                                             (9, 3, 11, 1, 5, 1), (70, 64, 8, 1, 3, 1), (40, 80, 9, 3, 1, 1)])
+@pytest.mark.parametrize("w_zp,in_zp", [(120, 128), (-9, -5)])
+def test_large_windows_of_asymmetric_weights(ctx, port, H, C, k, s, pad, dil, w_zp, in_zp):
+    """Window sums inside the product and in a launch of their own, on both sides of the line between them, in memory of the
+    plan's and of the caller's, and after the zero points have changed."""
+    import torch
+    t = np.int8 if in_zp < 0 else np.uint8
+    rng = np.random.default_rng(H * C + k)
+    B, OFM = 2, 24
+    src, wgt = q8_uniform(rng, (B, H, H, C), t), q8_uniform(rng, (OFM, k, k, C), t)
+    bias = rng.integers(-500, 501, OFM).astype(np.int32)
+    mult, shift = f32_mults(port, 0.03, np.array([4e-3], np.float32), 0.03 * np.sqrt(k * k * C))
+    lo, hi = type_range(t)
+    code = capi.S8 if t == np.int8 else capi.U8
+
+    def desc_for(izp, wzp):
+        return capi.make_conv_desc(B, H, H, C, OFM, k, k, (s, s), (pad,) * 4, (dil, dil), code, code, izp, wzp, multiplier=int(mult[0]), shift=int(shift[0]),
+                                   dst_zp=5, min_bound=lo, max_bound=hi, has_bias=True)
+    d_src, d_w, d_b = (torch.from_numpy(x.view(np.uint8) if x.dtype != np.int32 else x).cuda() for x in (src, wgt, bias))
+    for implicit, bind in ((True, False), (True, True), (False, True)):
+        desc, keep = desc_for(in_zp, w_zp)
+        plan = capi.ConvPlan(ctx, desc, keep)
+        plan.allow_implicit(implicit)
+        guard, n = 256, plan.temp_bytes
+        ws = torch.full((guard + n + guard,), 0x77, dtype=torch.uint8, device="cuda")
+        if bind:
+            plan.bind_temp(ws[guard:], n)
+        plan.prepare(d_w)
+        wo, ho = plan.out_dims()
+        d_dst = torch.empty((B, ho, wo, OFM), dtype=torch.uint8, device="cuda")
+        for izp, wzp in ((in_zp, w_zp), (in_zp + 2, w_zp + 3)):
+            if (izp, wzp) != (in_zp, w_zp):
+                plan.update_quantization(*desc_for(izp, wzp))
+            plan.run(d_src, d_b, d_dst)
+            plan.run(d_src, d_b, d_dst)
+            ctx.sync()
+            want = port.conv2d_nhwc(src, wgt, bias, (s, s), (pad,) * 4, izp, wzp, mult, shift, 5, lo, hi, (dil, dil))
+            assert np.array_equal(d_dst.cpu().numpy().view(t), want), (implicit, bind, izp)
+        assert (ws[:guard] == 0x77).all() and (ws[guard + n:] == 0x77).all()
+        plan.close()
+
+
 @pytest.mark.parametrize("geom", [(16, 56, 56, 1, 64, 128), (13, 57, 59, 1, 40, 0), (11, 60, 61, 1, 64, 0), (50, 57, 59, 2, 64, 7)])
 def test_double_tile_conv_vs_oracle(ctx, port, geom):
     """3x3 x 64 convolutions large enough (more than 256 output pixels per SM) for the gather kernel's 256-pixel units,
