@@ -839,7 +839,7 @@ __device__ __forceinline__ void flush_stage_many(const uint8_t *stage, const Til
 // A call of its own: inlined, its addresses cost the drain of aligned rows registers.
 // Rows of at most kShortRow bytes that lie close together: a lane writes the row it has staged, byte by byte (a warp then fills whole
 // sectors; a wider pitch, as the last group of a wide row has, belongs to the words).  Spread over the lanes as words they took
-// longer than their bytes' way to memory: 100000 x 17 x 256 13.4 / 11.3 us, 20000 x 9 x 64 6.8 / 6.4 (x 31 still 6.8 / 6.7).
+// longer than their bytes' way to memory: 100000 x 17 x 256 13.4 / 11.4 us, 20000 x 9 x 64 6.8 / 6.4.
 // d0: first valid byte of row 0 in global memory; rows, n: valid rows and bytes per row (at most kOutRowBytes).
 // tma: the stage is in the tensor map's swizzle (dst would take bulk stores, it is the residual whose rows are not aligned).
 __device__ __noinline__ void flush_stage_words(const uint8_t *__restrict__ stage, uint8_t *__restrict__ d0, int64_t ldd, int rows, int n,

@@ -129,8 +129,9 @@ struct ConvOperands
 };
 // Filter taps up to which the implicit kernel adds up the windows of pixel sums itself (window_sum: nine loads at a time, per
 // tile, behind the main loop's back); above, a launch of its own spreads them over the device, where the main loop is too short
-// to hide them (few channels, and up to 64 with few tiles).  Inside / apart, us: 1 x 14 x 14 x 16 -> 32 5 x 5 12.2 / 14, 7 x 7 17.1 / 12.2,
-// 11 x 11 32.8 / 16.2; 1 x 14 x 14 x 64 -> 32 7 x 7 17.6 / 18, 11 x 11 33.4 / 27.2; 8 x 28 x 28 x 128 -> 200 7 x 7 27.1 / 32.8.
+// to hide them (few channels, and up to 64 with few tiles).  Inside / apart, us: 1 x 14 x 14 x 16 -> 32 7 x 7 17.1 / 12.2,
+// 11 x 11 32.8 / 16.2, 1 x 14 x 14 x 64 -> 32 11 x 11 33.4 / 27.2; 1 x 14 x 14 x 128 -> 32 7 x 7 21.9 / 23.7, 8 x 28 x 28 x 64 -> 200 23.5 / 25.3,
+// x 128 27.1 / 32.8.  (25 taps are three rounds of loads; 5 x 5 inside is level with or ahead of the explicit lowering.)
 constexpr int kWindowTaps = 25;
 // out[m] = sum over the kh x kw window of output pixel m of the pixel sums, out-of-image taps counting cv.pad_sum
 cugl_status launch_window_sums(cugl_context *ctx, const int32_t *d_pixel_sums, const ConvOperands &cv, int M, int32_t *d_out);
